@@ -13,7 +13,7 @@ LIB = os.path.join(HERE, "libffxcuda.so")
 PEAK_SRC = "peak.cu"
 PEAK_LIB = os.path.join(HERE, "libffxpeak.so")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
-              "-Xcompiler", "-fPIC", "-shared", "-diag-suppress", "177"]
+              "-Xcompiler", "-fPIC", "-shared", "-diag-suppress", "177", "--threads", "8"]
 
 
 def nvcc() -> str:
@@ -27,7 +27,7 @@ def stale() -> bool:
     if not os.path.exists(LIB):
         return True
     t = os.path.getmtime(LIB)
-    deps = [os.path.join(HERE, "csrc", s) for s in SOURCES + ["ffx_internal.cuh"]]
+    deps = [os.path.join(HERE, "csrc", s) for s in SOURCES + ["ffx_internal.cuh", "launch.cuh", "fft.cuh"]]
     deps.append(os.path.join(os.path.dirname(HERE), "include", "ffxcuda.h"))
     return any(os.path.getmtime(d) > t for d in deps)
 

@@ -22,9 +22,8 @@
 // recordings cannot be merged.
 //
 // Results are those of the single-system path: the same bodies run on the same buffers
-// with the same grids.  (A system with a 64 x 64 mixed-form mesh takes the per-axis FFT
-// passes inside a stage-by-stage batch instead of its four-CTA cluster passes: the same
-// transform, rounded differently.)
+// with the same grids (the FFT passes with their own block size: each item's arithmetic is
+// the same).
 #include <algorithm>
 #include <cstring>
 #include <map>

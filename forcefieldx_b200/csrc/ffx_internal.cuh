@@ -353,6 +353,26 @@ struct FftAxis {
   int radix[12];
 };
 
+// Division of a block's item index by a run-time constant n: m = ceil(2^32 / n).
+struct FastDiv {
+  unsigned m;
+  int n;
+};
+
+// One axis of the two-step FFT (fft.cuh): n = f1 f2, f1 <= f2 <= 16.
+struct FftLine {
+  int n, f1, f2;
+  FastDiv by_n, by_f1, by_f2;
+};
+
+// A mesh's plan: the axes, and how many rows (forward) or columns (inverse) a plane's CTA
+// takes along its first axis at a time.
+struct FftPlan {
+  FftLine line[3];
+  int row_chunk, col_chunk;
+  FastDiv by_row_chunk, by_col_chunk;
+};
+
 // Device-side state of the PCG solve (read by the host after the loop).
 struct PcgState {
   double eps;     // last convergence measure, Debye
@@ -498,18 +518,20 @@ struct Handle {
   double *h_scalars = nullptr;                // pinned mirror
   // PME
   int nfft[3] = {0, 0, 0};
-  double2 *d_grid = nullptr;
+  double2 *d_grid = nullptr;                  // accumulation mesh: real plane, then imaginary plane
+  double2 *d_gridd = nullptr;                 // FP64 form: the complex mesh of the FFT and interpolation
   double *d_influence = nullptr;
   double2 *d_twiddle = nullptr;               // per-axis twiddle tables (3 x max n)
   // Mixed form: d_spl holds float data; spreading accumulates (exactly) in the double
-  // mesh d_grid and the FFT and interpolation run on the FP32 mesh d_gridf.
+  // planes of d_grid and the FFT and interpolation run on the FP32 mesh d_gridf.
   float2 *d_gridf = nullptr;
   float *d_influencef = nullptr;
   float2 *d_twiddlef = nullptr;
-  // The mixed form's accumulation mesh as two planes of doubles (real, imaginary).
   double *d_grid_planes() const { return reinterpret_cast<double *>(d_grid); }
   PmeConst pc{};
   FftAxis axes[3]{};
+  FftPlan fft_plan{};
+  bool fft_planned = false;                   // whether the axes and shared memory allow it
 
   // ---- outputs
   double *d_grad = nullptr, *d_torque = nullptr;  // [3][n]

@@ -228,15 +228,16 @@ static double charge_correction(const Handle &h, double q) {
 // is released first).
 static int alloc_mesh(Handle &h) {
   for (void *q : {(void *)h.d_grid, (void *)h.d_influence, (void *)h.d_twiddle, (void *)h.d_gridf,
-                  (void *)h.d_influencef, (void *)h.d_twiddlef})
+                  (void *)h.d_gridd, (void *)h.d_influencef, (void *)h.d_twiddlef})
     if (q) cudaFree(q);
   h.d_grid = nullptr; h.d_influence = nullptr; h.d_twiddle = nullptr;
-  h.d_gridf = nullptr; h.d_influencef = nullptr; h.d_twiddlef = nullptr;
+  h.d_gridf = nullptr; h.d_gridd = nullptr; h.d_influencef = nullptr; h.d_twiddlef = nullptr;
   const int nfx = h.prm.pme_grid[0], nfy = h.prm.pme_grid[1], nfz = h.prm.pme_grid[2];
   const size_t ng = (size_t)nfx * nfy * nfz;
   CK(dalloc(&h.d_grid, ng)); CK(dalloc(&h.d_influence, ng));
-  CK(cudaMemset(h.d_grid, 0, ng * sizeof(double2)));   // the mixed form keeps it clear between uses
+  CK(cudaMemset(h.d_grid, 0, ng * sizeof(double2)));   // the first FFT pass keeps it clear between uses
   CK(dalloc(&h.d_twiddle, 3 * (size_t)std::max(nfx, std::max(nfy, nfz))));
+  if (!h.mixed) CK(dalloc(&h.d_gridd, ng));
   if (h.mixed) {
     CK(dalloc(&h.d_gridf, ng));
     CK(dalloc(&h.d_influencef, ng));
@@ -584,7 +585,7 @@ static void free_all(Handle &h) {
                   h.d_nbr_cnt, h.d_nbl, h.d_nbl_cnt, h.d_ewl, h.d_ewl_cnt, h.d_prl, h.d_prl_cnt, h.d_gm, h.d_fm, h.d_spl, h.d_igrid,
                   h.d_cphi, h.d_fphi, h.d_cphiI, h.d_fphiI, h.d_cphiP, h.d_fphiP, h.d_fieldD, h.d_fieldP, h.d_uD,
                   h.d_uP, h.d_udirD, h.d_udirP, h.d_r, h.d_rP, h.d_zpre, h.d_zpreP, h.d_p, h.d_pP, h.d_vec, h.d_vecP,
-                  h.d_partials, h.d_scalars, h.d_grid, h.d_influence, h.d_twiddle, h.d_gridf, h.d_influencef, h.d_twiddlef, h.d_grad, h.d_torque, h.d_gred,
+                  h.d_partials, h.d_scalars, h.d_grid, h.d_influence, h.d_twiddle, h.d_gridf, h.d_gridd, h.d_influencef, h.d_twiddlef, h.d_grad, h.d_torque, h.d_gred,
                   h.d_eatom, h.d_catom, h.d_result, h.d_cresult, h.d_flags, h.d_xyz_in, h.d_grad_out,
                   h.d_coefE, h.d_coefP, h.d_coefEB, h.d_coefPB, h.d_part2, h.d_counter, h.d_pos, h.d_rpos, h.d_erec, h.d_recF, h.d_recP, h.d_tpair, h.d_tp, h.d_soft, h.d_mol, h.d_lgred, h.d_mass, h.d_mdx, h.d_mdv, h.d_mda, h.d_mdxp, h.d_mdg, h.d_mdke, h.d_settle, h.d_aspc, h.d_aspc_state, h.d_nbr_sh, h.d_ewl_sh, h.d_lg, h.d_lt, h.d_acc, h.d_polar_env, h.d_lig, h.d_rot};
   for (void *q : ptrs)
@@ -1662,6 +1663,7 @@ static int build_vacuum(Handle &h, const std::vector<int> &soft, const std::vect
   // gradient stay zero.
   const size_t ng = (size_t)vh.nfft[0] * vh.nfft[1] * vh.nfft[2];
   VK(cudaMemset(vh.d_grid, 0, ng * sizeof(double2)));
+  if (vh.d_gridd) VK(cudaMemset(vh.d_gridd, 0, ng * sizeof(double2)));
   if (vh.d_gridf) VK(cudaMemset(vh.d_gridf, 0, ng * sizeof(float2)));
   for (double *q : {vh.d_cphi, vh.d_fphi, vh.d_cphiI, vh.d_fphiI, vh.d_cphiP, vh.d_fphiP})
     VK(cudaMemset(q, 0, 20 * M * sizeof(double)));

@@ -5,23 +5,21 @@
 //  k_bsplines         ReciprocalSpace.BSplineLoop (ReciprocalSpace.java:1338-1412), UniformBSpline (:98-183),
 //                     toFractionalMultipole (:1212-1236)
 //  k_spread_*         SpatialPermanentLoop / SpatialInducedLoop (ReciprocalSpace.java:1445-1505, 1573-1628)
-//  k_fft_axis         Complex3DParallel.convolution (N/fft/Complex3DParallel.java:445, 775-795, 972-1010):
-//                     X and Y passes, a fused Z pass (FFT, influence function, inverse FFT), inverse Y, X.
+//  k_fft_plane, k_fft_z (fft.cuh), k_fft_axis
+//                     Complex3DParallel.convolution (N/fft/Complex3DParallel.java:445, 775-795, 972-1010):
+//                     X and Y, a fused Z pass (FFT, influence function, inverse FFT), inverse Y, X.
 //  k_phi              PermanentPhiLoop / InducedPhiLoop (ReciprocalSpace.java:2295-2454, 2506-2775)
 //
-// The mesh is one interleaved complex double grid [nz][ny][nx], 16 B per point, kept
-// L2-resident between passes.  Spreading uses FP64 atomics into the mesh.
+// Spreading adds into two planes of doubles with FP64 atomics; the transforms run on an
+// interleaved complex mesh [nz][ny][nx] of the form's type.  Both stay in L2 between passes.
 #include <atomic>
 #include <cmath>
 #include <cstring>
 #include <map>
 #include <mutex>
 
-#include <cooperative_groups.h>
-
 #include "ffx_internal.cuh"
-
-namespace cg = cooperative_groups;
+#include "fft.cuh"
 
 namespace ffx {
 
@@ -207,32 +205,26 @@ __device__ __forceinline__ int jmod(int a, int m) {
   return r < 0 ? r + m : r;
 }
 
-// Mesh accumulation with FP64 atomics.  FP64 form: into the complex double mesh that the
-// FFT transforms in place.  Mixed form: into two planes of doubles (real parts, then
-// imaginary parts, ng points each), so that a warp's row of five support points touches
-// two 32-byte sectors instead of three; each FP32 contribution is first rounded to a
-// multiple of 2^-32, so sums of such values are exact in FP64 (below 2^21 in magnitude)
-// and the accumulated mesh has the same bits whatever order the atoms arrive in.  The
-// first FFT pass reads the planes and continues in FP32.
+// Mesh accumulation with FP64 atomics into two planes of doubles (real parts, then
+// imaginary parts, ng points each), so that a warp's row of five support points touches two
+// 32-byte sectors per plane instead of three of an interleaved mesh; the first FFT pass
+// reads the planes and clears them.  Mixed form: each FP32 contribution is first rounded to
+// a multiple of 2^-32, so sums of such values are exact in FP64 (below 2^21 in magnitude)
+// and the accumulated mesh has the same bits whatever order the atoms arrive in.
 __device__ __forceinline__ double mesh_quantize(float v) {
   return rint((double)v * 4294967296.0) * 2.3283064365386962890625e-10;
 }
+__device__ __forceinline__ double mesh_quantize(double v) { return v; }
 // A mixed-form contribution of kQuantLimit or more raises FLAG_QUANT_RANGE (the first FFT
 // pass checks the accumulated values as it reads them).
-__device__ __forceinline__ void mesh_add(double2 *grid, size_t, size_t idx, double re, int *) {
-  atomicAdd(&grid[idx].x, re);
+template <typename S>
+__device__ __forceinline__ void mesh_add(double *plane, size_t idx, S re, int *flags) {
+  if (sizeof(S) == 4 && quant_out(re)) atomicOr(flags, FLAG_QUANT_RANGE);
+  atomicAdd(plane + idx, mesh_quantize(re));
 }
-__device__ __forceinline__ void mesh_add(double2 *grid, size_t, size_t idx, float re, int *flags) {
-  if (quant_out(re)) atomicOr(flags, FLAG_QUANT_RANGE);
-  atomicAdd(reinterpret_cast<double *>(grid) + idx, mesh_quantize(re));
-}
-__device__ __forceinline__ void mesh_add(double2 *grid, size_t, size_t idx, double re, double im, int *) {
-  atomicAdd(&grid[idx].x, re);
-  atomicAdd(&grid[idx].y, im);
-}
-__device__ __forceinline__ void mesh_add(double2 *grid, size_t ng, size_t idx, float re, float im, int *flags) {
-  if (quant_out(re) || quant_out(im)) atomicOr(flags, FLAG_QUANT_RANGE);
-  double *plane = reinterpret_cast<double *>(grid);
+template <typename S>
+__device__ __forceinline__ void mesh_add(double *plane, size_t ng, size_t idx, S re, S im, int *flags) {
+  if (sizeof(S) == 4 && (quant_out(re) || quant_out(im))) atomicOr(flags, FLAG_QUANT_RANGE);
   atomicAdd(plane + idx, mesh_quantize(re));
   atomicAdd(plane + ng + idx, mesh_quantize(im));
 }
@@ -245,13 +237,12 @@ __device__ __forceinline__ int wrap1(int v, int m) { return v < 0 ? v + m : (v >
 // the atomic add (no integer division in the loop).
 template <typename S>
 __device__ __forceinline__ void k_spread_permanent(VGrid vg, int n, const double *__restrict__ fm, const S *__restrict__ spl,
-                                   const int *__restrict__ igrid, int nfx, int nfy, int nfz, double2 *grid,
+                                   const int *__restrict__ igrid, int nfx, int nfy, int nfz, double *plane,
                                    int *flags) {
   const int warp = (vg.bid * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= n || lane >= 25) return;
   const int i = warp;
-  const size_t ng = (size_t)nfx * nfy * nfz;
   const S *s = spl + (size_t)i * 3 * kOrder * 4;
   const S *sx = s, *sy = s + kOrder * 4, *sz = s + 2 * kOrder * 4;
   const int a1 = lane % 5, a2 = lane / 5;
@@ -274,7 +265,7 @@ __device__ __forceinline__ void k_spread_permanent(VGrid vg, int n, const double
     const S term2 = f[t200] * v0 * u0;
     const S val = fma(x0, term0, fma(x1, term1, x2 * term2));
     const int kk = wrap1(k0 + a3, nfz);
-    mesh_add(grid, ng, (size_t)kk * nfy * nfx + row, val, flags);
+    mesh_add(plane, (size_t)kk * nfy * nfx + row, val, flags);
   }
 }
 
@@ -282,7 +273,7 @@ template <typename S>
 __device__ __forceinline__ void k_spread_induced(
     VGrid vg, int const &n, const double *__restrict__ const &ud, const double *__restrict__ const &up,
     const S *__restrict__ const &spl, const int *__restrict__ const &igrid, int const &nfx, int const &nfy,
-    int const &nfz, double2 * const &grid, const PmeConst &pc, int * const &flags) {
+    int const &nfz, double * const &plane, const PmeConst &pc, int * const &flags) {
   const int warp = (vg.bid * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= n || lane >= 25) return;
@@ -313,7 +304,7 @@ __device__ __forceinline__ void k_spread_induced(
     const S re = fma(v0, Ad, v1 * Bd);
     const S im = fma(v0, Ap, v1 * Bp);
     const int kk = wrap1(k0 + a3, nfz);
-    mesh_add(grid, ng, (size_t)kk * nfy * nfx + row, re, im, flags);
+    mesh_add(plane, ng, (size_t)kk * nfy * nfx + row, re, im, flags);
   }
 }
 
@@ -333,15 +324,7 @@ __device__ __forceinline__ V2 cmul(V2 a, V2 b) {
 // Radix-R Stockham butterfly for one (line, j) pair.  R is a compile-time constant so
 // the R values stay in registers; the small DFTs of R = 2, 3, 4 use their closed
 // forms, R = 5 and 7 use the twiddle table.
-// The twiddle table tw is in global memory (GTW: read through the read-only path) or in
-// shared memory (the fixed-length kernels).
-template <typename V2, bool GTW>
-__device__ __forceinline__ V2 tw_at(const V2 *tw, int i) {
-  if constexpr (GTW) return __ldg(tw + i);
-  else return tw[i];
-}
-
-template <int R, typename S, bool GTW = false>
+template <int R, typename S>
 __device__ __forceinline__ void fft_butterfly(const typename Vec2<S>::type *in, typename Vec2<S>::type *out, int j,
                                               int l, int L, int nb, int Ns, int len, int sg,
                                               const typename Vec2<S>::type *__restrict__ tw) {
@@ -353,7 +336,7 @@ __device__ __forceinline__ void fft_butterfly(const typename Vec2<S>::type *in, 
   for (int r = 0; r < R; r++) {
     V2 a = in[(j + r * nb) * L + l];
     if (r > 0 && k > 0) {
-      V2 w = tw_at<V2, GTW>(tw, r * k * tstep);
+      V2 w = __ldg(tw + r * k * tstep);
       if (sg > 0) w.y = -w.y;
       a = cmul(a, w);
     }
@@ -391,7 +374,7 @@ __device__ __forceinline__ void fft_butterfly(const typename Vec2<S>::type *in, 
       V2 acc = v[0];
 #pragma unroll
       for (int r = 1; r < R; r++) {
-        V2 w = tw_at<V2, GTW>(tw, ((r * q) % R) * wstep);
+        V2 w = __ldg(tw + ((r * q) % R) * wstep);
         if (sg > 0) w.y = -w.y;
         const V2 m = cmul(v[r], w);
         acc.x += m.x; acc.y += m.y;
@@ -406,7 +389,7 @@ __device__ __forceinline__ void fft_butterfly(const typename Vec2<S>::type *in, 
 // Radix-R pass for any R known only at run time (prime factors above 7, as the general
 // pass of Complex.java:173-330 handles them): each output q of the length-R DFT is summed
 // from the R twiddled inputs read from shared memory, O(R^2) per butterfly.
-template <typename S, bool GTW = false>
+template <typename S>
 __device__ __forceinline__ void fft_butterfly_any(int R, const typename Vec2<S>::type *in,
                                                   typename Vec2<S>::type *out, int j, int l, int L, int nb, int Ns,
                                                   int len, int sg, const typename Vec2<S>::type *__restrict__ tw) {
@@ -420,11 +403,11 @@ __device__ __forceinline__ void fft_butterfly_any(int R, const typename Vec2<S>:
     for (int r = 1; r < R; r++) {
       V2 a = in[(j + r * nb) * L + l];
       if (k > 0) {
-        V2 w = tw_at<V2, GTW>(tw, r * k * tstep);
+        V2 w = __ldg(tw + r * k * tstep);
         if (sg > 0) w.y = -w.y;
         a = cmul(a, w);
       }
-      V2 w = tw_at<V2, GTW>(tw, ((r * q) % R) * wstep);
+      V2 w = __ldg(tw + ((r * q) % R) * wstep);
       if (sg > 0) w.y = -w.y;
       a = cmul(a, w);
       acc.x += a.x;
@@ -434,9 +417,9 @@ __device__ __forceinline__ void fft_butterfly_any(int R, const typename Vec2<S>:
   }
 }
 
-// FROMD (mixed form, first pass only): the input is the double accumulation mesh `src`
-// (real plane, then imaginary plane at src + src_ng), converted to FP32 on load and
-// cleared behind the read, so that the next spread starts from zero without a memset.
+// FROMD (first pass only): the input is the double accumulation mesh `src` (real plane,
+// then imaginary plane at src + src_ng), cleared behind the read, so that the next spread
+// starts from zero without a memset.
 template <bool FUSE_G, typename S, bool FROMD>
 __device__ __forceinline__ void k_fft_axis(VGrid vg, typename Vec2<S>::type *grid, const FftAxis &ax, int sign,
                                                   const typename Vec2<S>::type *__restrict__ tw,
@@ -458,7 +441,7 @@ __device__ __forceinline__ void k_fft_axis(VGrid vg, typename Vec2<S>::type *gri
     const size_t g = base + (size_t)l * ax.line_step + (size_t)j * ax.stride;
     if (FROMD) {
       const double2 q = make_double2(src[g], src[src_ng + g]);
-      if (quant_out(q.x) || quant_out(q.y)) atomicOr(flags, FLAG_QUANT_RANGE);
+      if (sizeof(S) == 4 && (quant_out(q.x) || quant_out(q.y))) atomicOr(flags, FLAG_QUANT_RANGE);
       src[g] = 0.0;
       src[src_ng + g] = 0.0;
       buf0[j * L + l] = mk2<S>((S)q.x, (S)q.y);
@@ -478,12 +461,12 @@ __device__ __forceinline__ void k_fft_axis(VGrid vg, typename Vec2<S>::type *gri
       for (int t = threadIdx.x; t < nb * L; t += blockDim.x) {
         const int l = t % L, j = t / L;
         switch (R) {
-          case 4: fft_butterfly<4, S, true>(in, out, j, l, L, nb, Ns, len, sg, tw); break;
-          case 2: fft_butterfly<2, S, true>(in, out, j, l, L, nb, Ns, len, sg, tw); break;
-          case 3: fft_butterfly<3, S, true>(in, out, j, l, L, nb, Ns, len, sg, tw); break;
-          case 5: fft_butterfly<5, S, true>(in, out, j, l, L, nb, Ns, len, sg, tw); break;
-          case 7: fft_butterfly<7, S, true>(in, out, j, l, L, nb, Ns, len, sg, tw); break;
-          default: fft_butterfly_any<S, true>(R, in, out, j, l, L, nb, Ns, len, sg, tw); break;
+          case 4: fft_butterfly<4, S>(in, out, j, l, L, nb, Ns, len, sg, tw); break;
+          case 2: fft_butterfly<2, S>(in, out, j, l, L, nb, Ns, len, sg, tw); break;
+          case 3: fft_butterfly<3, S>(in, out, j, l, L, nb, Ns, len, sg, tw); break;
+          case 5: fft_butterfly<5, S>(in, out, j, l, L, nb, Ns, len, sg, tw); break;
+          case 7: fft_butterfly<7, S>(in, out, j, l, L, nb, Ns, len, sg, tw); break;
+          default: fft_butterfly_any<S>(R, in, out, j, l, L, nb, Ns, len, sg, tw); break;
         }
       }
       __syncthreads();
@@ -503,184 +486,6 @@ __device__ __forceinline__ void k_fft_axis(VGrid vg, typename Vec2<S>::type *gri
   }
   for (int t = threadIdx.x; t < len * L; t += blockDim.x) {
     const int l = contiguous ? t / len : t % L, j = contiguous ? t % len : t / L;
-    grid[base + (size_t)l * ax.line_step + (size_t)j * ax.stride] = in[j * L + l];
-  }
-}
-
-// Fixed-length line FFT (length LEN known at compile time, L lines per CTA, 256
-// threads).  The same Stockham passes as k_fft_axis, but every index division is by a
-// constant and the twiddle table sits in shared memory: at 64^3 the runtime-length
-// kernel spends most of its issue slots on integer division.
-__host__ __device__ constexpr int plan_radix(int len, int st) {
-  int m = len;
-  const int f[5] = {4, 2, 3, 5, 7};
-  for (int q = 0; q < 5; q++)
-    while (m % f[q] == 0) {
-      if (st == 0) return f[q];
-      st--;
-      m /= f[q];
-    }
-  return 0;
-}
-
-// LS: the element stride of the shared layout (L, or L + 1 to spread a line's elements
-// over the banks when lines are loaded along their elements).
-template <int LEN, int ST, int NS, int L, typename S, int LS = L>
-__device__ __forceinline__ void fixed_stages(typename Vec2<S>::type *&in, typename Vec2<S>::type *&out,
-                                             const typename Vec2<S>::type *tw, int sg) {
-  constexpr int R = plan_radix(LEN, ST);
-  if constexpr (R != 0) {
-    constexpr int NB = LEN / R;
-    for (int t = threadIdx.x; t < NB * L; t += 256) {
-      const int l = t % L, j = t / L;
-      fft_butterfly<R, S>(in, out, j, l, LS, NB, NS, LEN, sg, tw);
-    }
-    __syncthreads();
-    typename Vec2<S>::type *tmp = in;
-    in = out;
-    out = tmp;
-    fixed_stages<LEN, ST + 1, NS * R, L, S, LS>(in, out, tw, sg);
-  }
-}
-
-// Two-dimensional FFT of the 64 x 64 (x, y) planes of an FP32 mesh by a cluster of four
-// CTAs per z plane.  Forward: CTA c transforms rows y in [16c, 16c + 16) along x, the
-// cluster synchronises, and CTA c gathers columns x in [16c, 16c + 16) of every row from
-// the four CTAs' shared memory and transforms them along y.  Inverse: the same with the
-// axes swapped (y first, then x).  Two mesh passes become one launch, and the exchange
-// between them stays on chip.  FROMD (forward only): the input is the planar double
-// accumulation mesh (real plane, imaginary plane at + src_ng), which is cleared behind
-// the read so that the next spread starts from zero.
-template <bool INVERSE, bool FROMD>
-__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256)
-    k_fft_plane64(float2 *grid, int sign, const float2 *__restrict__ twg, double *src, size_t src_ng, int *flags) {
-  constexpr int LEN = 64, L = 16, LS = L + 1, NP = LEN * L, NB = LEN * LS, PER = NP / 256;
-  __shared__ float2 buf[3][NB];
-  __shared__ float2 tw[LEN];
-  cg::cluster_group cluster = cg::this_cluster();
-  const int c = (int)cluster.block_rank();
-  const size_t plane = (size_t)(blockIdx.x >> 2) * LEN * LEN;
-  for (int t = threadIdx.x; t < LEN; t += 256) tw[t] = twg[t];
-  // Phase A lines: rows [16c, 16c + 16) along x (forward) or columns (inverse), stored
-  // element-major, line-minor with stride LS: a[j * LS + l].  All loads of a thread are
-  // issued before any store.
-  {
-    float2 v[PER];
-    size_t g[PER];
-    int at[PER];
-#pragma unroll
-    for (int u = 0; u < PER; u++) {
-      const int t = threadIdx.x + 256 * u;
-      int j, l;
-      if (!INVERSE) {   // row l = t / 64, element x = t % 64 (coalesced rows)
-        l = t / LEN; j = t % LEN;
-        g[u] = plane + (size_t)(16 * c + l) * LEN + j;
-      } else {          // column x = 16c + t % 16, element y = t / 16
-        l = t % L; j = t / L;
-        g[u] = plane + (size_t)j * LEN + 16 * c + l;
-      }
-      at[u] = j * LS + l;
-      if (FROMD) {
-        const double re = src[g[u]], im = src[src_ng + g[u]];
-        if (quant_out(re) || quant_out(im)) atomicOr(flags, FLAG_QUANT_RANGE);
-        v[u] = make_float2((float)re, (float)im);
-      } else {
-        v[u] = grid[g[u]];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < PER; u++) {
-      if (FROMD) {
-        src[g[u]] = 0.0;
-        src[src_ng + g[u]] = 0.0;
-      }
-      buf[0][at[u]] = v[u];
-    }
-  }
-  __syncthreads();
-  float2 *in = buf[0], *out = buf[1];
-  fixed_stages<LEN, 0, 1, L, float, LS>(in, out, tw, sign);
-  // The first phase's result sits at the same offset in every CTA of the cluster.
-  const int res = (int)((in - &buf[0][0]) / NB);
-  const int spare = (res == 0) ? 1 : 0;
-  cluster.sync();
-  // Phase B lines: the other axis, gathered from the four CTAs into buf[2].  Forward:
-  // element y = j of column x = 16c + l lives in CTA y / 16 as its row y % 16, element x.
-  // Inverse: element x = j of row y = 16c + l lives in CTA x / 16 as its column x % 16,
-  // element y.  Both sit at [(16c + l) * LS + j % 16] of the owner.
-  {
-    float2 v[PER];
-#pragma unroll
-    for (int u = 0; u < PER; u++) {
-      const int t = threadIdx.x + 256 * u;
-      const int l = t % L, j = t / L;
-      const float2 *peer = cluster.map_shared_rank(&buf[res][0], j >> 4);
-      v[u] = peer[(16 * c + l) * LS + (j & 15)];
-    }
-#pragma unroll
-    for (int u = 0; u < PER; u++) {
-      const int t = threadIdx.x + 256 * u;
-      buf[2][(t / L) * LS + t % L] = v[u];
-    }
-  }
-  cluster.sync();   // every peer has read this CTA's phase-A result
-  in = buf[2];
-  out = buf[spare];
-  fixed_stages<LEN, 0, 1, L, float, LS>(in, out, tw, sign);
-  for (int t = threadIdx.x; t < NP; t += 256) {
-    size_t g;
-    int j, l;
-    if (!INVERSE) {   // column x = 16c + t % 16, element y = t / 16
-      l = t % L; j = t / L;
-      g = plane + (size_t)j * LEN + 16 * c + l;
-    } else {          // row y = 16c + t / 64, element x = t % 64
-      l = t / LEN; j = t % LEN;
-      g = plane + (size_t)(16 * c + l) * LEN + j;
-    }
-    grid[g] = in[j * LS + l];
-  }
-}
-
-template <int LEN, int L, bool FUSE_G, typename S, bool FROMD>
-__device__ __forceinline__ void k_fft_fixed(VGrid vg, typename Vec2<S>::type *grid, const FftAxis &ax, int sign,
-                                                   const typename Vec2<S>::type *__restrict__ twg,
-                                                   const S *__restrict__ G, int gnx, int gny,
-                                                   double *src, size_t src_ng, int *flags) {
-  using V2 = typename Vec2<S>::type;
-  __shared__ V2 buf[2][LEN * L];
-  __shared__ V2 tw[LEN];
-  for (int t = threadIdx.x; t < LEN; t += 256) tw[t] = twg[t];
-  const int gi = vg.bid % ax.groups_inner, go = vg.bid / ax.groups_inner;
-  const size_t base = (size_t)gi * ax.group_step_inner + (size_t)go * ax.group_step_outer;
-  const bool contiguous = (ax.stride == 1);
-  for (int t = threadIdx.x; t < LEN * L; t += 256) {
-    const int l = contiguous ? t / LEN : t % L, j = contiguous ? t % LEN : t / L;
-    const size_t g = base + (size_t)l * ax.line_step + (size_t)j * ax.stride;
-    if (FROMD) {
-      const double2 q = make_double2(src[g], src[src_ng + g]);
-      if (quant_out(q.x) || quant_out(q.y)) atomicOr(flags, FLAG_QUANT_RANGE);
-      src[g] = 0.0;
-      src[src_ng + g] = 0.0;
-      buf[0][j * L + l] = mk2<S>((S)q.x, (S)q.y);
-    } else {
-      buf[0][j * L + l] = grid[g];
-    }
-  }
-  __syncthreads();
-  V2 *in = buf[0], *out = buf[1];
-  fixed_stages<LEN, 0, 1, L, S>(in, out, tw, sign);
-  if (FUSE_G) {
-    for (int t = threadIdx.x; t < LEN * L; t += 256) {
-      const int l = t % L, j = t / L;
-      const S gv = G[(size_t)j * gnx * gny + base + (size_t)l * ax.line_step];
-      in[j * L + l].x *= gv;
-      in[j * L + l].y *= gv;
-    }
-    __syncthreads();
-    fixed_stages<LEN, 0, 1, L, S>(in, out, tw, -sign);
-  }
-  for (int t = threadIdx.x; t < LEN * L; t += 256) {
-    const int l = contiguous ? t / LEN : t % L, j = contiguous ? t % LEN : t / L;
     grid[base + (size_t)l * ax.line_step + (size_t)j * ax.stride] = in[j * L + l];
   }
 }
@@ -860,11 +665,10 @@ static FftAxis make_axis(int axis, const int nf[3]) {
   }
   // Lines of a CTA: consecutive along the fastest index that is not the transform axis;
   // up to 1,024 elements for short lines (a whole plane of a small mesh per CTA, so that
-  // the 256 threads have work in every stage), else 16 lines.  Length 64 keeps 16: the
-  // fixed-length kernel takes exactly that shape.
+  // the 256 threads have work in every stage), else 16 lines.
   const int inner = (axis == 0) ? ny : nx;
   int L = 1;
-  const int cap = (a.len == 64) ? 16 : std::max(1, std::max(std::min(16, 4096 / a.len), std::min(64, 1024 / a.len)));
+  const int cap = std::max(1, std::max(std::min(16, 4096 / a.len), std::min(64, 1024 / a.len)));
   for (int d = 1; d <= cap; d++)
     if (inner % d == 0) L = d;
   a.L = L;
@@ -913,17 +717,110 @@ struct FftAxisPass {
   }
 };
 
+// The two-step passes (fft.cuh), likewise.
+template <typename S, bool INV, bool WIDE>
+struct FftPlanePass {
+  using V = typename Vec2<S>::type;
+  static constexpr int T = fft_plane_threads<S, WIDE>(), B = fft_plane_blocks<S, WIDE>();
+  static void launch(Handle &h, int block, size_t smem, V *mesh, const FftPlan &pl, const V *tw, int tw_step,
+                     double *src, size_t ng) {
+    launch_on<k_fft_plane<S, INV, WIDE>, T, B>(h.rec, pl.line[2].n, block, smem, h.stream, mesh, pl, tw, tw_step, src,
+                                               ng, h.d_flags);
+  }
+  static cudaError_t raise(int need) {
+    const cudaError_t e1 =
+        cudaFuncSetAttribute(one_fn<k_fft_plane<S, INV, WIDE>, T, B, V *, FftPlan, const V *, int, double *, size_t, int *>(),
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, need);
+    const cudaError_t e2 =
+        cudaFuncSetAttribute(many_fn<k_fft_plane<S, INV, WIDE>, T, B, V *, FftPlan, const V *, int, double *, size_t, int *>(),
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, need);
+    return e1 != cudaSuccess ? e1 : e2;
+  }
+};
+template <typename S, bool WIDE>
+struct FftZPass {
+  using V = typename Vec2<S>::type;
+  static void launch(Handle &h, int blocks, int block, size_t smem, V *mesh, const FftPlan &pl, const V *tw,
+                     int tw_step, const S *G) {
+    launch_on<k_fft_z<S, WIDE>, 256, 0>(h.rec, blocks, block, smem, h.stream, mesh, pl, tw, tw_step, G);
+  }
+  static cudaError_t raise(int need) {
+    const cudaError_t e1 = cudaFuncSetAttribute(one_fn<k_fft_z<S, WIDE>, 256, 0, V *, FftPlan, const V *, int, const S *>(),
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize, need);
+    const cudaError_t e2 = cudaFuncSetAttribute(many_fn<k_fft_z<S, WIDE>, 256, 0, V *, FftPlan, const V *, int, const S *>(),
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize, need);
+    return e1 != cudaSuccess ? e1 : e2;
+  }
+};
+
+template <typename S>
+static cudaError_t raise_fft_smem_of(int need) {
+  const cudaError_t e[9] = {FftAxisPass<false, S, false>::raise(need), FftAxisPass<false, S, true>::raise(need),
+                            FftAxisPass<true, S, false>::raise(need),  FftPlanePass<S, false, false>::raise(need),
+                            FftPlanePass<S, false, true>::raise(need), FftPlanePass<S, true, false>::raise(need),
+                            FftPlanePass<S, true, true>::raise(need),  FftZPass<S, false>::raise(need),
+                            FftZPass<S, true>::raise(need)};
+  for (cudaError_t q : e)
+    if (q != cudaSuccess) return q;
+  return cudaSuccess;
+}
+
 static cudaError_t raise_fft_smem(int device, int need) {
   std::lock_guard<std::mutex> lock(g_fft_smem_mu);
   int &cur = g_fft_smem[device];
   if (need <= cur) return cudaSuccess;
-  const cudaError_t e[5] = {FftAxisPass<false, double, false>::raise(need), FftAxisPass<true, double, false>::raise(need),
-                            FftAxisPass<false, float, false>::raise(need), FftAxisPass<false, float, true>::raise(need),
-                            FftAxisPass<true, float, false>::raise(need)};
+  const cudaError_t e[2] = {raise_fft_smem_of<double>(need), raise_fft_smem_of<float>(need)};
   for (cudaError_t q : e)
     if (q != cudaSuccess) return q;
   cur = need;
   return cudaSuccess;
+}
+
+static FastDiv fast_div(int n) { return {(unsigned)(((1ull << 32) + n - 1) / n), n}; }
+
+// n = f1 f2 with factors the register DFTs cover, the larger as small as it goes; false
+// when there is none (a prime factor above 7, or n beyond 256).
+static bool fft_line(int n, FftLine &a) {
+  static const int radix[] = {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 15, 16};
+  a = FftLine{};
+  for (int f2 : radix) {
+    if (n % f2 || n / f2 > f2) continue;
+    for (int f1 : radix)
+      if (f1 * f2 == n) {
+        a.n = n; a.f1 = f1; a.f2 = f2;
+        a.by_n = fast_div(n); a.by_f1 = fast_div(f1); a.by_f2 = fast_div(f2);
+        return true;
+      }
+  }
+  return false;
+}
+
+static size_t fft_plane_smem(const FftPlan &p, size_t value) {
+  const FftLine &x = p.line[0], &y = p.line[1];
+  const size_t RS = (size_t)(x.f1 * (x.f2 | 1)) | 1, CS = (size_t)(y.f1 * (y.f2 | 1)) | 1;
+  return (std::max(p.row_chunk * RS + x.n * CS, y.n * RS + p.col_chunk * CS) + x.n + y.n) * value;
+}
+static size_t fft_z_smem(const FftPlan &p, size_t value) { return (2 * (size_t)kFftZLines + 1) * p.line[2].n * value; }
+
+// Whether the mesh takes the two-step passes: every axis has its two factors and a plane
+// fits one CTA's shared memory (FP32 up to about 150 x 150, FP64 100 x 100).  The first
+// axis goes in one chunk where that fits 160 KB, so that a plane has four barriers, and
+// else in as few as fit.
+static bool plan_fft(const int nf[3], size_t value, FftPlan &p) {
+  p = FftPlan{};
+  for (int d = 0; d < 3; d++)
+    if (!fft_line(nf[d], p.line[d])) return false;
+  constexpr size_t kMax = 227 * 1024;
+  size_t limit = 160 * 1024;
+  for (int parts = 1; parts <= 16; parts++) {
+    p.row_chunk = (nf[1] + parts - 1) / parts;
+    p.col_chunk = (nf[0] + parts - 1) / parts;
+    p.by_row_chunk = fast_div(p.row_chunk);
+    p.by_col_chunk = fast_div(p.col_chunk);
+    if (fft_plane_smem(p, value) <= limit) return fft_z_smem(p, value) <= kMax;
+    if (parts == 8) limit = kMax;
+  }
+  return false;
 }
 
 // Dynamic shared memory of one generic FFT pass over axis a (both sizes of the mesh type
@@ -1029,8 +926,11 @@ int setup_pme(Handle &h) {
     cudaMemcpy(h.d_twiddlef, twf.data(), twf.size() * sizeof(float2), cudaMemcpyHostToDevice);
   }
   for (int d = 0; d < 3; d++) h.axes[d] = make_axis(d, nf);
+  const size_t value = h.mixed ? sizeof(float2) : sizeof(double2);
+  h.fft_planned = plan_fft(nf, value, h.fft_plan);
   size_t smem = 48 * 1024;
   for (int d = 0; d < 3; d++) smem = std::max(smem, fft_axis_smem(h.axes[d]));
+  if (h.fft_planned) smem = std::max(smem, std::max(fft_plane_smem(h.fft_plan, value), fft_z_smem(h.fft_plan, value)));
   if (smem > 227 * 1024) {
     h.err = "PME grid dimension too long for the shared-memory FFT";
     return FFXG_ERR_BAD_ARG;
@@ -1066,48 +966,50 @@ void launch_bsplines(Handle &h) {
 
 static size_t grid_points(const Handle &h) { return (size_t)h.nfft[0] * h.nfft[1] * h.nfft[2]; }
 
-// The FP64 mesh cleared before a spread.
-__device__ __forceinline__ void k_clear_mesh(VGrid vg, size_t m, double2 *grid) {
-  for (size_t j = (size_t)vg.bid * blockDim.x + threadIdx.x; j < m; j += (size_t)vg.nblk * blockDim.x)
-    grid[j] = make_double2(0.0, 0.0);
-}
-static void clear_mesh(Handle &h) {
-  const size_t m = grid_points(h);
-  launch_on<k_clear_mesh, 0, 0>(h.rec, (int)std::min<size_t>(nblocks((int64_t)m, 256), 4 * (size_t)h.num_sms), 256, 0,
-                                h.stream, m, h.d_grid);
-  FFX_LAUNCHED(h);
-}
-
-// Both forms accumulate into the double mesh d_grid; the FP64 form clears it first, the
-// mixed form keeps it clear between uses (its first FFT pass zeroes what it reads) and
-// continues in the FP32 mesh d_gridf.
+// Both forms accumulate into the planes of d_grid, which the first FFT pass zeroes as it
+// reads them, and continue in the complex mesh of the form (d_gridd or d_gridf).
 void launch_spread_permanent(Handle &h) {
   if (h.vacuum) return;   // no reciprocal space: the mesh and potentials stay zero
   const int nb = nblocks((int64_t)h.n * 32, 256);
-  if (!h.mixed) clear_mesh(h);
   if (h.mixed)
     launch_on<k_spread_permanent<float>, 0, 0>(h.rec, nb, 256, 0, h.stream, h.n, (const double *)h.d_fm,
                                                reinterpret_cast<const float *>(h.d_spl), (const int *)h.d_igrid,
-                                               h.nfft[0], h.nfft[1], h.nfft[2], h.d_grid, h.d_flags);
+                                               h.nfft[0], h.nfft[1], h.nfft[2], h.d_grid_planes(), h.d_flags);
   else
     launch_on<k_spread_permanent<double>, 0, 0>(h.rec, nb, 256, 0, h.stream, h.n, (const double *)h.d_fm,
                                                 (const double *)h.d_spl, (const int *)h.d_igrid, h.nfft[0],
-                                                h.nfft[1], h.nfft[2], h.d_grid, h.d_flags);
+                                                h.nfft[1], h.nfft[2], h.d_grid_planes(), h.d_flags);
   FFX_LAUNCHED(h);
 }
 
 void launch_spread_induced(Handle &h, const double *ud, const double *up) {
   if (h.vacuum) return;   // no reciprocal space: the mesh and potentials stay zero
   const int nb = nblocks((int64_t)h.n * 32, 256);
-  if (!h.mixed) clear_mesh(h);
   if (h.mixed)
     launch_on<k_spread_induced<float>, 0, 0>(h.rec, nb, 256, 0, h.stream, h.n, ud, up,
                                              reinterpret_cast<const float *>(h.d_spl), (const int *)h.d_igrid,
-                                             h.nfft[0], h.nfft[1], h.nfft[2], h.d_grid, h.pc, h.d_flags);
+                                             h.nfft[0], h.nfft[1], h.nfft[2], h.d_grid_planes(), h.pc,
+                                             h.d_flags);
   else
     launch_on<k_spread_induced<double>, 0, 0>(h.rec, nb, 256, 0, h.stream, h.n, ud, up, (const double *)h.d_spl,
-                                              (const int *)h.d_igrid, h.nfft[0], h.nfft[1], h.nfft[2], h.d_grid,
-                                              h.pc, h.d_flags);
+                                              (const int *)h.d_igrid, h.nfft[0], h.nfft[1], h.nfft[2],
+                                              h.d_grid_planes(), h.pc, h.d_flags);
+  FFX_LAUNCHED(h);
+}
+
+template <typename S, bool WIDE>
+static void fft_planes(Handle &h, const FftPlan &pl, typename Vec2<S>::type *mesh,
+                       const typename Vec2<S>::type *twiddle, bool inverse) {
+  const int step = std::max(h.nfft[0], std::max(h.nfft[1], h.nfft[2]));
+  const FftLine &x = pl.line[0], &y = pl.line[1];
+  const size_t smem = fft_plane_smem(pl, sizeof(typename Vec2<S>::type));
+  // A thread per item of the widest step (a batch's stages share one block size).
+  const int items = std::max(y.n * x.f2, x.n * y.f2);
+  const int block = h.rec ? 128 : std::min(fft_plane_threads<S, WIDE>(), (items + 31) / 32 * 32);
+  if (inverse)
+    FftPlanePass<S, true, WIDE>::launch(h, block, smem, mesh, pl, twiddle, step, nullptr, 0);
+  else
+    FftPlanePass<S, false, WIDE>::launch(h, block, smem, mesh, pl, twiddle, step, h.d_grid_planes(), grid_points(h));
   FFX_LAUNCHED(h);
 }
 
@@ -1117,9 +1019,23 @@ static void fft_convolution(Handle &h, typename Vec2<S>::type *grid, const typen
   using V = typename Vec2<S>::type;
   const int nfx = h.nfft[0], nfy = h.nfft[1], nfz = h.nfft[2];
   const int maxn = std::max(nfx, std::max(nfy, nfz));
-  // The mixed form's accumulation mesh: real plane, then imaginary plane.
+  if (h.fft_planned) {
+    const FftPlan &pl = h.fft_plan;
+    const bool wide = pl.line[0].f2 > 8 || pl.line[1].f2 > 8, wide_z = pl.line[2].f2 > 8;
+    if (wide) fft_planes<S, true>(h, pl, grid, twiddle, false);
+    else fft_planes<S, false>(h, pl, grid, twiddle, false);
+    const int blocks = (nfx * nfy + kFftZLines - 1) / kFftZLines;
+    const int block = h.rec ? 128 : std::min(256, (kFftZLines * pl.line[2].f2 + 31) / 32 * 32);
+    const size_t smem = fft_z_smem(pl, sizeof(V));
+    if (wide_z) FftZPass<S, true>::launch(h, blocks, block, smem, grid, pl, twiddle, maxn, influence);
+    else FftZPass<S, false>::launch(h, blocks, block, smem, grid, pl, twiddle, maxn, influence);
+    FFX_LAUNCHED(h);
+    if (wide) fft_planes<S, true>(h, pl, grid, twiddle, true);
+    else fft_planes<S, false>(h, pl, grid, twiddle, true);
+    return;
+  }
+  // Any other length (a prime factor above 7, or beyond 256): five per-axis passes.
   double *plane = h.d_grid_planes();
-  const size_t ng = (size_t)nfx * nfy * nfz;
   auto run = [&](int d, int sign, bool fuse, bool fromd) {
     const FftAxis &a = h.axes[d];
     const int outer = (d == 0) ? nfz : ((d == 1) ? nfz : nfy);
@@ -1127,43 +1043,15 @@ static void fft_convolution(Handle &h, typename Vec2<S>::type *grid, const typen
     const size_t smem = 2 * (size_t)a.len * a.L * sizeof(V);
     const V *tw = twiddle + (size_t)d * maxn;
     const S *none = nullptr;
-    if (a.len == 64 && a.L == 16) {
-      if (fuse)
-        launch_on<k_fft_fixed<64, 16, true, S, false>, 256, 0>(h.rec, blocks, 256, 0, h.stream, grid, a, sign, tw,
-                                                               influence, nfx, nfy, (double *)nullptr, (size_t)0,
-                                                               h.d_flags);
-      else if (fromd)
-        launch_on<k_fft_fixed<64, 16, false, S, true>, 256, 0>(h.rec, blocks, 256, 0, h.stream, grid, a, sign, tw,
-                                                               none, nfx, nfy, plane, ng, h.d_flags);
-      else
-        launch_on<k_fft_fixed<64, 16, false, S, false>, 256, 0>(h.rec, blocks, 256, 0, h.stream, grid, a, sign, tw,
-                                                                none, nfx, nfy, (double *)nullptr, (size_t)0,
-                                                                h.d_flags);
-      FFX_LAUNCHED(h);
-      return;
-    }
     if (fuse)
       FftAxisPass<true, S, false>::launch(h, blocks, smem, grid, a, sign, tw, influence, nfx, nfy, nullptr, 0);
     else if (fromd)
-      FftAxisPass<false, S, true>::launch(h, blocks, smem, grid, a, sign, tw, none, nfx, nfy, plane, ng);
+      FftAxisPass<false, S, true>::launch(h, blocks, smem, grid, a, sign, tw, none, nfx, nfy, plane, grid_points(h));
     else
       FftAxisPass<false, S, false>::launch(h, blocks, smem, grid, a, sign, tw, none, nfx, nfy, nullptr, 0);
     FFX_LAUNCHED(h);
   };
-  const bool fromd = (sizeof(S) == 4);   // mixed: the first pass reads the double mesh
-  if (sizeof(S) == 4 && nfx == 64 && nfy == 64 && h.axes[2].len == 64 && h.axes[2].L == 16 && !h.rec) {
-    // Mixed form on 64 x 64 planes: xy, z (with the influence function), yx.  (A recorded
-    // batch takes the per-axis passes instead: a cluster launch cannot span systems.)
-    float2 *gf = reinterpret_cast<float2 *>(grid);
-    const float2 *tw = reinterpret_cast<const float2 *>(twiddle);
-    k_fft_plane64<false, true><<<nfz * 4, 256, 0, h.stream>>>(gf, -1, tw, h.d_grid_planes(), ng, h.d_flags);
-    FFX_LAUNCHED(h);
-    run(2, -1, true, false);
-    k_fft_plane64<true, false><<<nfz * 4, 256, 0, h.stream>>>(gf, +1, tw, nullptr, 0, h.d_flags);
-    FFX_LAUNCHED(h);
-    return;
-  }
-  run(0, -1, false, fromd);
+  run(0, -1, false, true);
   run(1, -1, false, false);
   run(2, -1, true, false);
   run(1, +1, false, false);
@@ -1175,13 +1063,13 @@ void launch_fft_convolution(Handle &h) {
   if (h.mixed)
     fft_convolution<float>(h, h.d_gridf, h.d_twiddlef, h.d_influencef);
   else
-    fft_convolution<double>(h, h.d_grid, h.d_twiddle, h.d_influence);
+    fft_convolution<double>(h, h.d_gridd, h.d_twiddle, h.d_influence);
 }
 
 template <typename S>
 static void phi(Handle &h, int which) {
   const S *spl = reinterpret_cast<const S *>(h.d_spl);
-  const auto *grid = reinterpret_cast<const typename Vec2<S>::type *>(h.mixed ? (void *)h.d_gridf : (void *)h.d_grid);
+  const auto *grid = reinterpret_cast<const typename Vec2<S>::type *>(h.mixed ? (void *)h.d_gridf : (void *)h.d_gridd);
   const int nb = nblocks((int64_t)h.n * 32, 256);
   if (which == 0)
     launch_on<k_phi<20, S>, 256, 0, sizeof(S) == 4 ? 6 : 3>(h.rec, nb, 256, 0, h.stream, h.n, spl, (const int *)h.d_igrid, grid, h.nfft[0],

@@ -268,8 +268,7 @@ int ffxg_set_image_mode(ffxg_handle *h, int mode);
  * evaluation as a branch of one graph (GRAPH falls back to it when the systems'
  * evaluations cannot be merged into common stages); LOOP mode loops over single-system
  * launches, for comparison.  Results are those of the single-system path (bit for bit in
- * the mixed form, except a 64 x 64 mixed-form mesh, whose FFT a stage-by-stage batch
- * takes by its per-axis passes).
+ * the mixed form).
  *   systems[n_systems], params[n_systems]: as for ffxg_create, one per system.
  *   xyz, grad: all systems' coordinates / gradients concatenated in system order
  *     ([total atoms][3]; xyz may be NULL to reuse the last accepted coordinates;
