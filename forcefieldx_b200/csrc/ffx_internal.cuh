@@ -77,6 +77,7 @@ struct Box {
   double volume;
   double A10, A20, A21;    // off-diagonal terms of A (lower triangular)
   double Ai10, Ai20, Ai21; // off-diagonal terms of A^-1 (lower triangular)
+  float s00, s10, s20, s11, s21, s22;   // A^-1 / 2^32
   int tric;
 };
 
@@ -98,12 +99,29 @@ __device__ __forceinline__ void to_frac(double x, double y, double z, const Box 
   zf = __dmul_rn(z, bx.A22);
 }
 
+// -1 or +1, against the sign of v.
+__device__ __forceinline__ double minus_unit(double v) {
+  return __hiloint2double((__double2hiint(v) & 0x80000000) ^ 0xbff00000, 0);
+}
+
 __device__ __forceinline__ double image_exact(double &x, double &y, double &z, const Box &bx) {
   double xf, yf, zf;
   to_frac(x, y, z, bx, xf, yf, zf);
-  xf = __dadd_rn(__dmul_rn(floor(__dadd_rn(fabs(xf), 0.5)), jsignum(-xf)), xf);
-  yf = __dadd_rn(__dmul_rn(floor(__dadd_rn(fabs(yf), 0.5)), jsignum(-yf)), yf);
-  zf = __dadd_rn(__dmul_rn(floor(__dadd_rn(fabs(zf), 0.5)), jsignum(-zf)), zf);
+  // f + floor(|f| + 1/2) (-sign f).  Where |f| + 1/2 is below 2 the floor is 0 or 1 and the
+  // wrap is one exact addition of -+1, chosen by integer tests of the high words; the
+  // rounding and sign functions (a slow pipe, and most of this function's instructions) are
+  // left to fractions beyond that, infinities and NaN.
+  const double tx = __dadd_rn(fabs(xf), 0.5), ty = __dadd_rn(fabs(yf), 0.5), tz = __dadd_rn(fabs(zf), 0.5);
+  const int hx = __double2hiint(tx), hy = __double2hiint(ty), hz = __double2hiint(tz);
+  if (max(max(hx, hy), hz) < 0x40000000) {
+    if (hx >= 0x3ff00000) xf = __dadd_rn(xf, minus_unit(xf));
+    if (hy >= 0x3ff00000) yf = __dadd_rn(yf, minus_unit(yf));
+    if (hz >= 0x3ff00000) zf = __dadd_rn(zf, minus_unit(zf));
+  } else {
+    xf = __dadd_rn(__dmul_rn(floor(tx), jsignum(-xf)), xf);
+    yf = __dadd_rn(__dmul_rn(floor(ty), jsignum(-yf)), yf);
+    zf = __dadd_rn(__dmul_rn(floor(tz), jsignum(-zf)), zf);
+  }
   if (!bx.tric) {
     x = __dmul_rn(xf, bx.Ai00);
     y = __dmul_rn(yf, bx.Ai11);
@@ -166,6 +184,74 @@ __device__ __forceinline__ bool pair_counted(int i, int k, const int *__restrict
   const int c = sh[e];
   const int nx = (c & 1023) - 512, ny = ((c >> 10) & 1023) - 512, nz = ((c >> 20) & 1023) - 512;
   return nz > 0 || (nz == 0 && (ny > 0 || (ny == 0 && nx > 0)));
+}
+
+// Fractional coordinates as 32-bit fixed point: a difference of two wraps to the minimum
+// image by itself.
+__device__ __forceinline__ int4 fixed_fraction(double x, double y, double z, const Box &bx) {
+  double xf, yf, zf;
+  to_frac(x, y, z, bx, xf, yf, zf);
+  return make_int4((int)__double2ll_rn(xf * 4294967296.0), (int)__double2ll_rn(yf * 4294967296.0),
+                   (int)__double2ll_rn(zf * 4294967296.0), 0);
+}
+
+// r^2 of the minimum image from fixed-point fractions, in FP32: within 1e-5 relative of the
+// exact one for any pair closer than half the cell.
+__device__ __forceinline__ float fixed_r2(const int4 &a, const int4 &b, const Box &bx) {
+  const float fx = (float)(int)((unsigned)a.x - (unsigned)b.x), fy = (float)(int)((unsigned)a.y - (unsigned)b.y);
+  const float fz = (float)(int)((unsigned)a.z - (unsigned)b.z);
+  float x = fx * bx.s00, y = fy * bx.s11;
+  const float z = fz * bx.s22;
+  if (bx.tric) {
+    x = fmaf(fz, bx.s20, fmaf(fy, bx.s10, x));
+    y = fmaf(fz, bx.s21, y);
+  }
+  return fmaf(x, x, fmaf(y, y, z * z));
+}
+
+// A row scan tests r^2 <= cutoff^2 on the fixed-point fractions first, against a bound this
+// much larger; what passes is tested exactly, in FP64, where it is worked on.
+__device__ __forceinline__ float scan_bound(double off2) { return (float)(off2 * 1.0001); }
+
+// Entries that pass a row scan, queued by the scanning warp and worked on 32 at a time: a
+// ring of kQueue (partner, place in the row), so that what stays behind after 32 need not
+// move.
+constexpr int kScan = 4, kQueue = 256;   // 32-entry chunks a scan step takes; slots (>= 31 + 32 kScan)
+struct PairQueue {
+  int2 e[kQueue];
+};
+
+// One step of a row scan by a warp: entries base .. base + 32 kScan - 1 of the row's m, the
+// loads of every chunk in flight together (a chunk at a time, the two dependent gathers are
+// most of a scan's time: vdW 158 us, against 137 with four).  The FP32 test costs a third of
+// the exact one's instructions, and nearly half of a buffered row fails it: vdW 195 -> 137 us
+// and the real-space field 154 -> 132 us on the 24,000-atom box, mixed form.  Appends what passes to the queue at `tail` and returns how many.
+// A multi-image row (sh set) lists shifts of the unwrapped coordinates: its entries all pass.
+__device__ __forceinline__ int scan_row(const int *__restrict__ row, int base, int m, const int4 &fi,
+                                        const int4 *__restrict__ fixed, const int *sh, const Box &bx, float bound,
+                                        int2 *queue, int tail) {
+  const int lane = threadIdx.x & 31;
+  int k[kScan], count = 0;
+  int4 f[kScan];
+#pragma unroll
+  for (int u = 0; u < kScan; u++) {
+    const int a = base + 32 * u + lane;
+    k[u] = a < m ? row[a] : -1;
+  }
+  if (!sh) {
+#pragma unroll
+    for (int u = 0; u < kScan; u++) f[u] = k[u] >= 0 ? __ldg(fixed + k[u]) : fi;
+  }
+#pragma unroll
+  for (int u = 0; u < kScan; u++) {
+    const bool pass = k[u] >= 0 && (sh || fixed_r2(f[u], fi, bx) <= bound);
+    const unsigned bal = __ballot_sync(0xffffffffu, pass);
+    if (pass)
+      queue[(tail + count + __popc(bal & ((1u << lane) - 1u))) & (kQueue - 1)] = make_int2(k[u], base + 32 * u + lane);
+    count += __popc(bal);
+  }
+  __syncwarp();
+  return count;
 }
 
 // Arithmetic of the two precision forms.  Pair kernels are templates on the pair-math
@@ -503,6 +589,7 @@ struct Handle {
   // dipoles of the PCG fields, [n][8] of double (plain) or float (mixed): d_recF holds
   // the dipoles whose field is taken (u, then p), d_recP holds alpha r.
   double2 *d_pos = nullptr;
+  int4 *d_ipos = nullptr, *d_irpos = nullptr;   // fixed-point fractions of x and of the reduced r
   void *d_recF = nullptr, *d_recP = nullptr;
   void *d_erec = nullptr;                     // [n][kRecStride] real-space gather records
   double2 *d_rpos = nullptr;                  // [n] (rx, ry), (rz, vdW type bits): vdW gather record
@@ -532,6 +619,7 @@ struct Handle {
   FftAxis axes[3]{};
   FftPlan fft_plan{};
   bool fft_planned = false;                   // whether the axes and shared memory allow it
+  int carve = 28;                             // shared-memory split of the kernels that run beside the mesh passes
 
   // ---- outputs
   double *d_grad = nullptr, *d_torque = nullptr;  // [3][n]

@@ -154,6 +154,13 @@ static int round32(double v) { return ((int)std::ceil(v) + 31) / 32 * 32; }
 // A their inverse (lower triangular: closed form), the volume and the perpendicular widths
 // 1 / |a*_d|, by the orthorhombic, monoclinic (only beta differs from 90) and general
 // branches.  Angles of 0 read as 90.
+// The lattice vectors over 2^32, the steps of the fixed-point fractions.
+static void set_steps(Box &b) {
+  const double q = 1.0 / 4294967296.0;
+  b.s00 = (float)(b.Ai00 * q); b.s10 = (float)(b.Ai10 * q); b.s20 = (float)(b.Ai20 * q);
+  b.s11 = (float)(b.Ai11 * q); b.s21 = (float)(b.Ai21 * q); b.s22 = (float)(b.Ai22 * q);
+}
+
 static Box make_box(const double box[3], const double angles[3], double width[3]) {
   Box b{};
   b.a = box[0]; b.b = box[1]; b.c = box[2];
@@ -165,6 +172,7 @@ static Box make_box(const double box[3], const double angles[3], double width[3]
     b.volume = b.a * b.b * b.c;
     b.tric = 0;
     width[0] = b.a; width[1] = b.b; width[2] = b.c;
+    set_steps(b);
     return b;
   }
   const double deg = 0.017453292519943295;   // Math.toRadians
@@ -191,6 +199,7 @@ static Box make_box(const double box[3], const double angles[3], double width[3]
   width[0] = 1.0 / std::sqrt(b.A00 * b.A00 + b.A10 * b.A10 + b.A20 * b.A20);
   width[1] = 1.0 / std::sqrt(b.A11 * b.A11 + b.A21 * b.A21);
   width[2] = 1.0 / std::fabs(b.A22);
+  set_steps(b);
   return b;
 }
 
@@ -483,6 +492,7 @@ static int create_impl(const ffxg_system *s, const ffxg_params *p, Handle &h) {
   CK(dalloc(&h.d_r, 3 * N)); CK(dalloc(&h.d_rP, 3 * N)); CK(dalloc(&h.d_zpre, 3 * N)); CK(dalloc(&h.d_zpreP, 3 * N));
   CK(dalloc(&h.d_p, 3 * N)); CK(dalloc(&h.d_pP, 3 * N));
   CK(dalloc(&h.d_pos, 2 * N)); CK(dalloc(&h.d_rpos, 2 * N));
+  CK(dalloc(&h.d_ipos, N)); CK(dalloc(&h.d_irpos, N));
   CK(cudaMalloc(&h.d_erec, (size_t)kRecStride * N * sizeof(double)));
   CK(cudaMemset(h.d_erec, 0, (size_t)kRecStride * N * sizeof(double)));
   CK(dalloc(&h.d_tpair, 6 * N)); CK(dalloc(&h.d_tp, 6 * N));
@@ -587,7 +597,7 @@ static void free_all(Handle &h) {
                   h.d_uP, h.d_udirD, h.d_udirP, h.d_r, h.d_rP, h.d_zpre, h.d_zpreP, h.d_p, h.d_pP, h.d_vec, h.d_vecP,
                   h.d_partials, h.d_scalars, h.d_grid, h.d_influence, h.d_twiddle, h.d_gridf, h.d_gridd, h.d_influencef, h.d_twiddlef, h.d_grad, h.d_torque, h.d_gred,
                   h.d_eatom, h.d_catom, h.d_result, h.d_cresult, h.d_flags, h.d_xyz_in, h.d_grad_out,
-                  h.d_coefE, h.d_coefP, h.d_coefEB, h.d_coefPB, h.d_part2, h.d_counter, h.d_pos, h.d_rpos, h.d_erec, h.d_recF, h.d_recP, h.d_tpair, h.d_tp, h.d_soft, h.d_mol, h.d_lgred, h.d_mass, h.d_mdx, h.d_mdv, h.d_mda, h.d_mdxp, h.d_mdg, h.d_mdke, h.d_settle, h.d_aspc, h.d_aspc_state, h.d_nbr_sh, h.d_ewl_sh, h.d_lg, h.d_lt, h.d_acc, h.d_polar_env, h.d_lig, h.d_rot};
+                  h.d_coefE, h.d_coefP, h.d_coefEB, h.d_coefPB, h.d_part2, h.d_counter, h.d_pos, h.d_rpos, h.d_ipos, h.d_irpos, h.d_erec, h.d_recF, h.d_recP, h.d_tpair, h.d_tp, h.d_soft, h.d_mol, h.d_lgred, h.d_mass, h.d_mdx, h.d_mdv, h.d_mda, h.d_mdxp, h.d_mdg, h.d_mdke, h.d_settle, h.d_aspc, h.d_aspc_state, h.d_nbr_sh, h.d_ewl_sh, h.d_lg, h.d_lt, h.d_acc, h.d_polar_env, h.d_lig, h.d_rot};
   for (void *q : ptrs)
     if (q) cudaFree(q);
   if (h.h_scalars) cudaFreeHost(h.h_scalars);
@@ -674,14 +684,22 @@ static void emit_front(Handle &h, const double *d_xyz) {
   launch_set_coordinates(h, d_xyz);
   launch_neighbor_list(h, false);
   timer_end(h, tk);
-  if (h.capturing && !h.vacuum && !h.batch_branch) {
-    // A branch of the graph: vdW depends on the list alone, and only the gradient
-    // assembly and the sums read it (emit_back joins it there).  Inside a batch graph the
-    // systems are the branches, and vdW stays in line (measured 16% more systems/s).
-    cudaEventRecord(h.ev_vdw_fork, h.stream);
+  // In a captured evaluation vdW, which needs the list alone and which only the gradient
+  // assembly and the sums read (emit_back joins it there), is a branch of the graph.  Before
+  // a solve it starts after the real-space field: beside the solver it takes idle issue
+  // slots, beside the field it takes the field's (172 against 132 us on the 24,000-atom box,
+  // mixed form; 354 against 220 us FP64).  Inside a batch graph the systems are the branches,
+  // and vdW stays in line (measured 16% more systems/s).
+  const bool vdw_branch = h.capturing && !h.vacuum && !h.batch_branch;
+  const bool vdw_late = vdw_branch && h.prm.polarization == FFXG_POLAR_MUTUAL;
+  auto fork_vdw = [&](cudaStream_t from) {
+    cudaEventRecord(h.ev_vdw_fork, from);
     cudaStreamWaitEvent(h.vdw_stream, h.ev_vdw_fork, 0);
     launch_vdw(h, h.want_grad, h.vdw_stream);
     cudaEventRecord(h.ev_vdw_join, h.vdw_stream);
+  };
+  if (vdw_branch) {
+    if (!vdw_late) fork_vdw(h.stream);
   } else {
     tk = timer_begin(h, FFXG_STAGE_VDW);
     launch_vdw(h, h.want_grad, h.stream);
@@ -713,8 +731,24 @@ static void emit_front(Handle &h, const double *d_xyz) {
     timer_end(h, tk);
   }
   tk = timer_begin(h, FFXG_STAGE_PERM_FIELD);
-  launch_realspace_field(h);   // sub-lists, permanent real-space field, pair coefficients
-  if (branch_recip(h)) cudaStreamWaitEvent(h.stream, h.ev_recip_join, 0);
+  // Sub-lists, permanent real-space field, pair coefficients: on the low-priority stream
+  // where the reciprocal chain is a branch, so that the chain's small launches are placed
+  // as the field's blocks retire instead of after them.
+  if (branch_recip(h)) {
+    cudaEventRecord(h.ev_fork, h.stream);
+    cudaStreamWaitEvent(h.aux, h.ev_fork, 0);
+    cudaStream_t main = h.stream;
+    h.stream = h.aux;
+    launch_realspace_field(h);
+    h.stream = main;
+    cudaEventRecord(h.ev_join, h.aux);
+    if (vdw_late) fork_vdw(h.aux);
+    cudaStreamWaitEvent(h.stream, h.ev_join, 0);
+    cudaStreamWaitEvent(h.stream, h.ev_recip_join, 0);
+  } else {
+    launch_realspace_field(h);
+    if (vdw_late) fork_vdw(h.stream);
+  }
   launch_direct_dipoles(h);
   timer_end(h, tk);
 }

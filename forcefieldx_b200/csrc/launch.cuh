@@ -187,4 +187,28 @@ inline void launch_on(Recorder *rec, int grid, int block, size_t smem, cudaStrea
   else k_one<BODY, MAXT, MINB, A...><<<grid, block, smem, st>>>(a...);
 }
 
+// As launch_on, with a preferred shared-memory carve-out (percent of the SM's largest) for
+// the single-system launch.  An SM's split between L1 and shared memory is fixed while
+// blocks are resident, and a kernel that wants a larger one waits for them to end: kernels
+// that run beside each other name the same split.
+template <auto BODY, int MAXT, int MINB, int MB = MINB, typename... A>
+inline void launch_split_on(Recorder *rec, int carve, int grid, int block, size_t smem, cudaStream_t st, const A &...a) {
+  if (rec) {
+    launch_on<BODY, MAXT, MINB, MB>(rec, grid, block, smem, st, a...);
+    return;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  at[0].val.sharedMemCarveout = (unsigned)carve;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  void *args[] = {const_cast<void *>(static_cast<const void *>(&a))...};
+  cudaLaunchKernelExC(&cfg, one_fn<BODY, MAXT, MINB, A...>(), args);
+}
+
 }  // namespace ffx

@@ -16,35 +16,29 @@ struct CellOffsets {
   int off[3][5];
 };
 
-// Interleaved [n][3] -> SoA, plus reduced coordinates r = a*(x - x_p) + x_p evaluated
-// without contraction like Java (VanDerWaals.java:1521-1527).
+// Interleaved [n][3] -> SoA and gather records, the reduced coordinates r = a*(x - x_p) + x_p
+// evaluated without contraction like Java (VanDerWaals.java:1521-1527), the motion and
+// reduction-offset checks, and the fixed-point fractions that the row scans test first.
 __device__ __forceinline__ void k_set_coordinates(VGrid vg, int n, const double *__restrict__ xyz, const int *__restrict__ redp,
                                   const double *__restrict__ redf, double *x, double *y, double *z,
-                                  double *rx, double *ry, double *rz, double2 *pos) {
+                                  double *rx, double *ry, double *rz, double2 *pos,
+                                  const double *__restrict__ refx, const double *__restrict__ refy,
+                                  const double *__restrict__ refz, double half_buffer2, int *flags,
+                                  const int *__restrict__ vtype, double2 *rpos, const Box &bx, int4 *ipos,
+                                  int4 *irpos) {
   const int i = vg.bid * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const double a = xyz[3 * i], b = xyz[3 * i + 1], c = xyz[3 * i + 2];
-  x[i] = a;
-  y[i] = b;
-  z[i] = c;
-  pos[2 * i] = make_double2(a, b);
-  pos[2 * i + 1] = make_double2(c, 0.0);
-}
-
-__device__ __forceinline__ void k_reduce_coordinates(VGrid vg, int n, const double *__restrict__ x, const double *__restrict__ y,
-                                     const double *__restrict__ z, const int *__restrict__ redp,
-                                     const double *__restrict__ redf, double *rx, double *ry, double *rz,
-                                     const double *__restrict__ refx, const double *__restrict__ refy,
-                                     const double *__restrict__ refz, double half_buffer2, int *flags,
-                                     const int *__restrict__ vtype, double2 *rpos) {
-  const int i = vg.bid * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  const double xi = xyz[3 * i], yi = xyz[3 * i + 1], zi = xyz[3 * i + 2];
   const int p = redp[i];
   const double a = redf[i];
-  const double xi = x[i], yi = y[i], zi = z[i];
+  x[i] = xi;
+  y[i] = yi;
+  z[i] = zi;
+  pos[2 * i] = make_double2(xi, yi);
+  pos[2 * i + 1] = make_double2(zi, 0.0);
   double vx = xi, vy = yi, vz = zi;
   if (p != i || a != 0.0) {
-    const double px = x[p], py = y[p], pz = z[p];
+    const double px = xyz[3 * p], py = xyz[3 * p + 1], pz = xyz[3 * p + 2];
     vx = __dadd_rn(__dmul_rn(a, __dsub_rn(xi, px)), px);
     vy = __dadd_rn(__dmul_rn(a, __dsub_rn(yi, py)), py);
     vz = __dadd_rn(__dmul_rn(a, __dsub_rn(zi, pz)), pz);
@@ -52,6 +46,8 @@ __device__ __forceinline__ void k_reduce_coordinates(VGrid vg, int n, const doub
   rx[i] = vx; ry[i] = vy; rz[i] = vz;
   rpos[2 * i] = make_double2(vx, vy);
   rpos[2 * i + 1] = make_double2(vz, __longlong_as_double((long long)vtype[i]));
+  ipos[i] = fixed_fraction(xi, yi, zi, bx);
+  irpos[i] = fixed_fraction(vx, vy, vz, bx);
   const double dx = vx - refx[i], dy = vy - refy[i], dz = vz - refz[i];
   const double d2 = dx * dx + dy * dy + dz * dz;
   if (!(d2 <= half_buffer2)) atomicOr(flags, FLAG_REBUILD);
@@ -341,15 +337,11 @@ __device__ __forceinline__ void k_cell_clear(VGrid vg, int m, int *cnt, const in
 // ---------------------------------------------------------------------------
 void launch_set_coordinates(Handle &h, const double *d_xyz) {
   const int n = h.n;
-  launch_on<k_set_coordinates, 0, 0>(h.rec, nblocks(n, 256), 256, 0, h.stream, n, d_xyz, (const int *)h.d_redp,
-                                     (const double *)h.d_redf, h.d_x, h.d_y, h.d_z, h.d_rx, h.d_ry, h.d_rz, h.d_pos);
-  FFX_LAUNCHED(h);
   const double hb = 0.5 * h.prm.list_buffer;
-  launch_on<k_reduce_coordinates, 0, 0>(h.rec, nblocks(n, 256), 256, 0, h.stream, n, (const double *)h.d_x,
-                                        (const double *)h.d_y, (const double *)h.d_z, (const int *)h.d_redp,
-                                        (const double *)h.d_redf, h.d_rx, h.d_ry, h.d_rz, (const double *)h.d_refx,
-                                        (const double *)h.d_refy, (const double *)h.d_refz, hb * hb, h.d_flags,
-                                        (const int *)h.d_vtype, h.d_rpos);
+  launch_on<k_set_coordinates, 0, 0>(h.rec, nblocks(n, 256), 256, 0, h.stream, n, d_xyz, (const int *)h.d_redp,
+                                     (const double *)h.d_redf, h.d_x, h.d_y, h.d_z, h.d_rx, h.d_ry, h.d_rz, h.d_pos,
+                                     (const double *)h.d_refx, (const double *)h.d_refy, (const double *)h.d_refz,
+                                     hb * hb, h.d_flags, (const int *)h.d_vtype, h.d_rpos, h.box, h.d_ipos, h.d_irpos);
   FFX_LAUNCHED(h);
 }
 

@@ -724,7 +724,7 @@ struct FftPlanePass {
   static constexpr int T = fft_plane_threads<S, WIDE>(), B = fft_plane_blocks<S, WIDE>();
   static void launch(Handle &h, int block, size_t smem, V *mesh, const FftPlan &pl, const V *tw, int tw_step,
                      double *src, size_t ng) {
-    launch_on<k_fft_plane<S, INV, WIDE>, T, B>(h.rec, pl.line[2].n, block, smem, h.stream, mesh, pl, tw, tw_step, src,
+    launch_split_on<k_fft_plane<S, INV, WIDE>, T, B>(h.rec, h.carve, pl.line[2].n, block, smem, h.stream, mesh, pl, tw, tw_step, src,
                                                ng, h.d_flags);
   }
   static cudaError_t raise(int need) {
@@ -742,7 +742,7 @@ struct FftZPass {
   using V = typename Vec2<S>::type;
   static void launch(Handle &h, int blocks, int block, size_t smem, V *mesh, const FftPlan &pl, const V *tw,
                      int tw_step, const S *G) {
-    launch_on<k_fft_z<S, WIDE>, 256, 0>(h.rec, blocks, block, smem, h.stream, mesh, pl, tw, tw_step, G);
+    launch_split_on<k_fft_z<S, WIDE>, 256, 0>(h.rec, h.carve, blocks, block, smem, h.stream, mesh, pl, tw, tw_step, G);
   }
   static cudaError_t raise(int need) {
     const cudaError_t e1 = cudaFuncSetAttribute(one_fn<k_fft_z<S, WIDE>, 256, 0, V *, FftPlan, const V *, int, const S *>(),
@@ -804,14 +804,17 @@ static size_t fft_z_smem(const FftPlan &p, size_t value) { return (2 * (size_t)k
 
 // Whether the mesh takes the two-step passes: every axis has its two factors and a plane
 // fits one CTA's shared memory (FP32 up to about 150 x 150, FP64 100 x 100).  The first
-// axis goes in one chunk where that fits 160 KB, so that a plane has four barriers, and
-// else in as few as fit.
+// axis goes in one chunk where that fits 100 KB, and else in as few as do (or as few as fit
+// at all): a chunk costs two barriers, a larger plane the L1 of the kernels beside it
+// (smem_split).  Device time of an evaluation with the limit at 160 / 120 / 100 / 60 KB:
+// 24,000 atoms FP64 2,042 / 1,787 / 1,799 / 1,899 us, 81,000 mixed 3,841 / 3,481 / 3,421 /
+// 3,553.
 static bool plan_fft(const int nf[3], size_t value, FftPlan &p) {
   p = FftPlan{};
   for (int d = 0; d < 3; d++)
     if (!fft_line(nf[d], p.line[d])) return false;
   constexpr size_t kMax = 227 * 1024;
-  size_t limit = 160 * 1024;
+  size_t limit = 100 * 1024;
   for (int parts = 1; parts <= 16; parts++) {
     p.row_chunk = (nf[1] + parts - 1) / parts;
     p.col_chunk = (nf[0] + parts - 1) / parts;
@@ -821,6 +824,16 @@ static bool plan_fft(const int nf[3], size_t value, FftPlan &p) {
     if (parts == 8) limit = kMax;
   }
   return false;
+}
+
+// The shared-memory split (percent of the SM's 228 KB) under which a plane's CTA and a vdW
+// block fit one SM: the smallest of the hardware's that does, since the rest is L1 for the
+// pair kernels' gathers.
+static int smem_split(size_t plane) {
+  const size_t need = plane + 8 * sizeof(PairQueue) + 3 * 1024;   // 1 KB of each block is the system's
+  for (int kb : {64, 100, 132, 164, 196})
+    if (need <= (size_t)kb * 1024) return (kb * 100 + 227) / 228;
+  return 100;
 }
 
 // Dynamic shared memory of one generic FFT pass over axis a (both sizes of the mesh type
@@ -928,6 +941,7 @@ int setup_pme(Handle &h) {
   for (int d = 0; d < 3; d++) h.axes[d] = make_axis(d, nf);
   const size_t value = h.mixed ? sizeof(float2) : sizeof(double2);
   h.fft_planned = plan_fft(nf, value, h.fft_plan);
+  h.carve = smem_split(h.fft_planned ? fft_plane_smem(h.fft_plan, value) : 0);
   size_t smem = 48 * 1024;
   for (int d = 0; d < 3; d++) smem = std::max(smem, fft_axis_smem(h.axes[d]));
   if (h.fft_planned) smem = std::max(smem, std::max(fft_plane_smem(h.fft_plan, value), fft_z_smem(h.fft_plan, value)));

@@ -44,13 +44,16 @@ struct Excl {
 };
 
 
-// Real-space lists, permanent real-space field and cached pair coefficients in one pass (PermanentRealSpaceFieldLoop, pme/PermanentFieldRegion.java:595-815, which also
-// derives the Ewald and preconditioner lists; DirectLoop, pme/DirectRegion.java:170-243).
-// Phase 1 compacts the buffered row into the Ewald row (r2 <= off2) and the
-// preconditioner row (r < pcut).  Phase 2 walks the Ewald row: it accumulates the D and
-// CR permanent fields and stores, per entry, the two symmetric coefficients of the
-// unmasked Thole-damped dipole field, A = bn1 - (1 - s3) rr3 and B = bn2 - (1 - s5) rr5,
-// so the field of any dipole set is -A u_k + B (u_k . r) r; entries inside the
+// Real-space lists, permanent real-space field and cached pair coefficients in one pass
+// (PermanentRealSpaceFieldLoop, pme/PermanentFieldRegion.java:595-815, which also derives the
+// Ewald and preconditioner lists; DirectLoop, pme/DirectRegion.java:170-243).  A warp scans
+// the buffered (or near) row of its atom; entries inside the cutoff
+// by a cheap FP32 test (fixed_r2) join a queue in shared memory and are worked on 32 at a
+// time, so that the exact minimum image, the FP64 test (r2 <= off2) and the pair arithmetic
+// run on full warps.  Per entry inside, the row gets the partner (the Ewald row), the D
+// and CR permanent fields are accumulated, and the two symmetric coefficients of the
+// unmasked Thole-damped dipole field are stored, A = bn1 - (1 - s3) rr3 and B = bn2 -
+// (1 - s5) rr5, so the field of any dipole set is -A u_k + B (u_k . r) r; entries inside the
 // preconditioner cutoff also store the Ewald-free pair (pme/PCGSolver.java:1300-1331).
 template <typename R>
 __device__ __forceinline__ void k_realspace_field(
@@ -64,7 +67,7 @@ __device__ __forceinline__ void k_realspace_field(
     const Excl &ex, const EwaldCoef &ec, const ScaleTables &c_scales, double * const &fieldD,
     double * const &fieldP, int * const &flags, const double2 *__restrict__ const &pos,
     const R *__restrict__ const &rec, const int *__restrict__ const &nbl, const int *__restrict__ const &nbl_cnt,
-    int const &capN) {
+    int const &capN, const int4 *__restrict__ const &ipos) {
   using V2 = typename Vec2<R>::type;
   const int warp = (vg.bid * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -72,73 +75,37 @@ __device__ __forceinline__ void k_realspace_field(
   const int i = warp;
   const unsigned lt = (1u << lane) - 1u;
   const double xi = x[i], yi = y[i], zi = z[i];
-  // ---- phase 1: sub-lists, from the near row when the near list is valid (every Ewald
-  // pair of this evaluation is in it), else from the buffered row
-  {
-    const bool nearrow = nbl && !(*flags & FLAG_NEAR_INVALID);
-    const int cnt = nearrow ? min(nbl_cnt[i], capN) : min(nbr_cnt[i], cap);
-    const int *row = nearrow ? nbl + (size_t)i * capN : nbr + (size_t)i * cap;
-    int ce = 0, cp = 0;
-    for (int base = 0; base < cnt; base += 32) {
-      const int a = base + lane;
-      bool ew = false, pr = false;
-      int k = -1;
-      if (a < cnt) {
-        k = row[a];
-        double xk, yk, zk;
-        load_pos(pos, k, xk, yk, zk);
-        double dx = __dsub_rn(xk, xi), dy = __dsub_rn(yk, yi), dz = __dsub_rn(zk, zi);
-        const double r2 = pair_image(dx, dy, dz, bx, nbr_sh, (size_t)i * cap + a, 1.0);
-        ew = r2 <= off2;
-        pr = ew && (r2 <= pcut2);   // sqrt(r2) < pcut, exactly (pcut2 from below_sqrt)
-      }
-      const unsigned me = __ballot_sync(0xffffffffu, ew);
-      const unsigned mp = __ballot_sync(0xffffffffu, pr);
-      if (ew) {
-        const int pos = ce + __popc(me & lt);
-        if (pos < capE) {
-          ewl[(size_t)i * capE + pos] = k;
-          if (nbr_sh) ewl_sh[(size_t)i * capE + pos] = nbr_sh[(size_t)i * cap + a];
-        }
-      }
-      if (pr) {
-        const int pos = cp + __popc(mp & lt);
-        if (pos < capP) prl[(size_t)i * capP + pos] = k;
-      }
-      ce += __popc(me);
-      cp += __popc(mp);
-    }
-    if (lane == 0) {
-      ewl_cnt[i] = ce;
-      prl_cnt[i] = cp;
-      if (ce > capE) atomicOr(flags, FLAG_EWALD_OVERFLOW);
-      if (cp > capP) atomicOr(flags, FLAG_PRECOND_OVERFLOW);
-    }
-  }
-  __syncwarp();
-  // ---- phase 2: permanent field and coefficients
+  __shared__ PairQueue qbuf[4];
+  int2 *queue = qbuf[threadIdx.x >> 5].e;
   const R pdi = ipdamp[i], pti = thole[i];
   const R aewald = ec.aewald, an0 = ec.an0, an1 = ec.an1, an2 = ec.an2;
   R fx = 0, fy = 0, fz = 0, px = 0, py = 0, pz = 0;
-  const int cnt = min(ewl_cnt[i], capE);
-  const int *row = ewl + (size_t)i * capE;
-  int cp = 0;
-  for (int base = 0; base < cnt; base += 32) {
-    const int a = base + lane;
-    const bool act = a < cnt;
-    bool pr = false;
-    R pA = R(0), pB = R(0), px_ = R(0), py_ = R(0), pz_ = R(0);
-    int pk = 0;
-    if (act) {
-      const int k = row[a];
-      const size_t ent = (size_t)i * capE + a;
+  int head = 0, done = 0, cp = 0;   // queue front, Ewald and preconditioner entries stored
+  // The queue's first m (m <= 32) entries.
+  auto work = [&](int m) {
+    bool ew = false, pr = false;
+    int k = 0, src = 0;
+    double xd = 0.0, yd = 0.0, zd = 0.0, r2d = 0.0;
+    if (lane < m) {
+      const int2 w = queue[(head + lane) & (kQueue - 1)];
+      k = w.x;
+      src = w.y;
       double xk, yk, zk;
       load_pos(pos, k, xk, yk, zk);
+      xd = __dsub_rn(xk, xi), yd = __dsub_rn(yk, yi), zd = __dsub_rn(zk, zi);
+      r2d = pair_image(xd, yd, zd, bx, nbr_sh, (size_t)i * cap + src, 1.0);
+      ew = r2d <= off2;
+    }
+    const unsigned me = __ballot_sync(0xffffffffu, ew);
+    const int a = done + __popc(me & lt);
+    R pA = R(0), pB = R(0), px_ = R(0), py_ = R(0), pz_ = R(0);
+    if (ew && a < capE) {
+      const size_t ent = (size_t)i * capE + a;
       R mk[12];
       load_rec<0, 12>(rec, k, mk);
-      double xd = __dsub_rn(xk, xi), yd = __dsub_rn(yk, yi), zd = __dsub_rn(zk, zi);
-      const double r2d = pair_image(xd, yd, zd, bx, ewl_sh, ent, 1.0);
       const R xr = (R)xd, yr = (R)yd, zr = (R)zd, r2 = (R)r2d;
+      ewl[ent] = k;
+      if (nbr_sh) ewl_sh[ent] = nbr_sh[(size_t)i * cap + src];
       const R ck = mk[t000], dkx = mk[t100], dky = mk[t010], dkz = mk[t001];
       const R qkxx = mk[t200], qkyy = mk[t020], qkzz = mk[t002], qkxy = mk[t110], qkxz = mk[t101], qkyz = mk[t011];
       const R r = m_sqrt(r2);
@@ -160,7 +127,7 @@ __device__ __forceinline__ void k_realspace_field(
         scale5 = R(1.0) - expdamp * (R(1.0) - damp);
         scale7 = R(1.0) - expdamp * (R(1.0) - damp + R(0.6) * damp * damp);
       }
-      const unsigned code = pair_primary(ewl_sh, ent) ? excl_code(i, k, ex.ptr, ex.k, ex.code, ex.lo, ex.hi) : 0u;
+      const unsigned code = pair_primary(nbr_sh, (size_t)i * cap + src) ? excl_code(i, k, ex.ptr, ex.k, ex.code, ex.lo, ex.hi) : 0u;
       const R scale = c_scales.d[(code >> 6) & 1u];
       const R scalep = c_scales.p[(code >> 3) & 7u];
       const R dsc3 = scale3 * scale, dsc5 = scale5 * scale, dsc7 = scale7 * scale;
@@ -189,28 +156,51 @@ __device__ __forceinline__ void k_realspace_field(
       px += fimx - fipx; py += fimy - fipy; pz += fimz - fipz;
       // Induced-field coefficients (no masks), InducedDipoleFieldRegion.java:383-404.
       const R urr3 = (R(1.0) - scale3) * rr3, urr5 = (R(1.0) - scale5) * rr5;
-      if (a < capE) {
-        store_pair(coefE, (size_t)i * capE + a, xr, yr, zr, bn1 - urr3);
-        store_pair_b(coefEB, (size_t)i * capE + a, k, bn2 - urr5);
-      }
-      pr = r2d <= pcut2;   // the same test, in FP64, that selected the preconditioner row
+      store_pair(coefE, ent, xr, yr, zr, bn1 - urr3);
+      store_pair_b(coefEB, ent, k, bn2 - urr5);
+      pr = r2d <= pcut2;   // sqrt(r2) < the preconditioner cutoff, exactly (pcut2 from below_sqrt)
       if (pr) {
         const R b1 = rr1 * rr2, b2 = R(3.0) * b1 * rr2;   // Ewald off: bn0 = 1/r
         pA = b1 - urr3;
         pB = b2 - urr5;
-        pk = k;
         px_ = xr; py_ = yr; pz_ = zr;
       }
     }
     const unsigned mp = __ballot_sync(0xffffffffu, pr);
     if (pr) {
-      const int pos = cp + __popc(mp & lt);
-      if (pos < capP) {
-        store_pair(coefP, (size_t)i * capP + pos, px_, py_, pz_, pA);
-        store_pair_b(coefPB, (size_t)i * capP + pos, pk, pB);
+      const int at = cp + __popc(mp & lt);
+      if (at < capP) {
+        prl[(size_t)i * capP + at] = k;
+        store_pair(coefP, (size_t)i * capP + at, px_, py_, pz_, pA);
+        store_pair_b(coefPB, (size_t)i * capP + at, k, pB);
       }
     }
     cp += __popc(mp);
+    done += __popc(me);
+    head += m;
+  };
+  // The near row when the near list is valid (every Ewald pair of this evaluation is in it),
+  // else the buffered row.
+  const bool nearrow = nbl && !(*flags & FLAG_NEAR_INVALID);
+  const int cnt = nearrow ? min(nbl_cnt[i], capN) : min(nbr_cnt[i], cap);
+  const int *row = nearrow ? nbl + (size_t)i * capN : nbr + (size_t)i * cap;
+  const int4 fi = ipos[i];
+  const float bound = scan_bound(off2);
+  int qn = 0;
+  for (int base = 0; base < cnt; base += 32 * kScan) {
+    qn += scan_row(row, base, cnt, fi, ipos, nbr_sh, bx, bound, queue, head + qn);
+    while (qn >= 32) {
+      work(32);
+      qn -= 32;
+    }
+    __syncwarp();
+  }
+  work(qn);
+  if (lane == 0) {
+    ewl_cnt[i] = done;
+    prl_cnt[i] = cp;
+    if (done > capE) atomicOr(flags, FLAG_EWALD_OVERFLOW);
+    if (cp > capP) atomicOr(flags, FLAG_PRECOND_OVERFLOW);
   }
   double Fx = warp_sum((double)fx), Fy = warp_sum((double)fy), Fz = warp_sum((double)fz);
   double Px = warp_sum((double)px), Py = warp_sum((double)py), Pz = warp_sum((double)pz);
@@ -769,8 +759,8 @@ static void realspace_field(Handle &h) {
                                    (const double *)h.d_ipdamp, (const double *)h.d_thole,
                                    reinterpret_cast<R *>(h.d_erec));
   FFX_LAUNCHED(h);
-  launch_on<k_realspace_field<R>, 128, sizeof(R) == 4 ? 8 : 1>(
-      h.rec, nblocks((int64_t)h.n * 32, 128), 128, 0, h.stream, h.n, (const double *)h.d_x, (const double *)h.d_y,
+  launch_split_on<k_realspace_field<R>, 128, sizeof(R) == 4 ? 8 : 1>(
+      h.rec, h.carve, nblocks((int64_t)h.n * 32, 128), 128, 0, h.stream, h.n, (const double *)h.d_x, (const double *)h.d_y,
       (const double *)h.d_z, h.box, (const double *)h.d_gm, (const double *)h.d_ipdamp, (const double *)h.d_thole,
       (const int *)h.d_nbr, (const int *)h.d_nbr_cnt, h.cap_nbr, (const int *)h.d_nbr_sh, off2,
       below_sqrt(h.prm.precond_cutoff), h.d_ewl, h.d_ewl_cnt, h.cap_ewl, h.d_ewl_sh, h.d_prl, h.d_prl_cnt, h.cap_prl,
@@ -778,7 +768,7 @@ static void realspace_field(Handle &h) {
       reinterpret_cast<PairRec<R> *>(h.d_coefP), reinterpret_cast<R *>(h.d_coefPB), excl(h),
       ewald_coef(h, ewald_alpha_of(h)), h.scales, h.d_fieldD, h.d_fieldP, h.d_flags, (const double2 *)h.d_pos,
       reinterpret_cast<const R *>(h.d_erec), (const int *)(h.near_list ? h.d_nbl : nullptr), (const int *)h.d_nbl_cnt,
-      h.cap_nbl);
+      h.cap_nbl, (const int4 *)h.d_ipos);
   FFX_LAUNCHED(h);
 }
 

@@ -4,9 +4,9 @@
 // (VanDerWaalsForm.java:313-334; delta 0.07, gamma 0.12), the multiplicative taper
 // from vdw-taper * cutoff to the cutoff (MultiplicativeSwitch.java:84-124, 234-236) and
 // the 1-2/1-3/1-4 masks (VanDerWaals.applyMask, :412-428).  A warp owns an atom i and
-// scans its buffered row in both directions (a partner's reduced position and type from
-// one 32-byte record); entries inside the cutoff go to a per-warp queue in shared memory
-// and are evaluated 32 at a time.  The force on i's reduced site accumulates in
+// scans its buffered row in both directions; entries inside the cutoff by an FP32 test on
+// fixed-point fractions go to a per-warp queue in shared memory and are evaluated 32 at a
+// time (a partner's reduced position and type from one 32-byte record).  The force on i's reduced site accumulates in
 // registers; k_vdw_distribute then splits every reduced-site force between the hydrogen
 // and its heavy atom (VanDerWaals.java:1786-1797) as a gather.
 #include <algorithm>
@@ -23,9 +23,7 @@ struct VdwForm {
 };
 
 __device__ __forceinline__ unsigned vexcl_code(int i, int k, const int *__restrict__ ptr, const int *__restrict__ ek,
-                                               const unsigned *__restrict__ code, const int *__restrict__ lo,
-                                               const int *__restrict__ hi) {
-  if (k < lo[i] || k > hi[i]) return 0u;
+                                               const unsigned *__restrict__ code) {
   const int e1 = ptr[i + 1];
   for (int e = ptr[i]; e < e1; e++)
     if (ek[e] == k) return code[e];
@@ -45,9 +43,8 @@ __device__ __forceinline__ void k_vdw(
     const ScaleTables &c_vscales, int const &gradient, double * const &eatom, long long * const &catom,
     double * const &gred, const int *__restrict__ const &soft, const int *__restrict__ const &mol,
     const AlchConst &al, double * const &edl, double * const &ed2l, double * const &lgred,
-    const double2 *__restrict__ const &rpos) {
-  struct Queue { R x[64], y[64], z[64], r[64], m[64]; int k[64], t[64], f[64]; };
-  __shared__ Queue qbuf[8];
+    const double2 *__restrict__ const &rpos, const int4 *__restrict__ const &irpos) {
+  __shared__ PairQueue qbuf[8];
   const int warp = (vg.bid * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int nwarps = (vg.nblk * blockDim.x) >> 5;
@@ -64,14 +61,34 @@ __device__ __forceinline__ void k_vdw(
     const int mol_i = ALCH ? mol[i] : 0;
     const int m = min(nbr_cnt[i], cap);
     const int *row = nbr + (size_t)i * cap;
-    // Entries inside the cutoff (with a non-zero mask) are queued in shared memory and
-    // evaluated 32 at a time, so the pair arithmetic runs on full warps instead of on the
-    // ~55% of lanes whose entry lies inside 9 A of an 11 A row.
-    R *qx = qbuf[wib].x, *qy = qbuf[wib].y, *qz = qbuf[wib].z, *qr = qbuf[wib].r, *qm = qbuf[wib].m;
-    int *qk = qbuf[wib].k, *qt = qbuf[wib].t, *qf = qbuf[wib].f;
-    auto pair_math = [&](int k, int tk, int qflags, R dx, R dy, R dz, R r2, R mask) {
-      const bool tap = (qflags & 1) != 0, counted = (qflags & 2) != 0;
+    // Entries inside the cutoff by a cheap FP32 test (fixed_r2) are queued in shared memory
+    // and worked on 32 at a time, so that the exact minimum image, the FP64 test and the pair
+    // arithmetic run on full warps instead of on the ~55% of lanes whose entry lies inside
+    // 9 A of an 11 A row.
+    int2 *queue = qbuf[wib].e;
+    const int lo = elo[i], hi = ehi[i];
+    const int4 fi = irpos[i];
+    const float bound = scan_bound(vf.off2);
+    int head = 0, qn = 0;
+    auto pair_math = [&]() {
+      const int2 qw = queue[(head + lane) & (kQueue - 1)];
+      const int k = qw.x;
+      const size_t ent = (size_t)i * cap + qw.y;
+      double pk[4];
+      ldg_32b(reinterpret_cast<const double *>(rpos + 2 * (size_t)k), pk);
+      double dxd = __dsub_rn(xi, pk[0]), dyd = __dsub_rn(yi, pk[1]), dzd = __dsub_rn(zi, pk[2]);
+      const double r2d = pair_image(dxd, dyd, dzd, bx, nbr_sh, ent, -1.0);
+      if (!(r2d <= vf.off2)) return;
+      R mask = R(1);
+      if (k >= lo && k <= hi && pair_primary(nbr_sh, ent)) {
+        mask = c_vscales.v[(vexcl_code(i, k, eptr, ek, ecode) >> 7) & 3u];
+        if (!(mask > R(0.0))) return;
+      }
+      const bool tap = r2d > vf.cut2, counted = pair_counted(i, k, nbr_sh, ent);
+      const R dx = (R)dxd, dy = (R)dyd, dz = (R)dzd, r2 = (R)r2d;
+      const int tk = (int)__double_as_longlong(pk[3]);
       const R irv = vrad[ti * ntypes + tk];
+      if (!(irv > R(0.0))) return;   // types that do not interact
         const R r = m_sqrt(r2);
         // Softcore pair (VanDerWaals.java:1728-1761): exactly one atom soft, or both soft under
         // the intermolecular / intramolecular softcore options.
@@ -166,49 +183,17 @@ __device__ __forceinline__ void k_vdw(
           }
         }
     };
-    int qn = 0;
-    for (int base = 0; base < m; base += 32) {
-      const int a = base + lane;
-      bool pass = false;
-      int k = 0, tk = 0, qflags = 0;
-      R dx = 0, dy = 0, dz = 0, r2 = 0, mask = 0;
-      if (a < m) {
-        k = row[a];
-        const size_t ent = (size_t)i * cap + a;
-        double pk[4];
-        ldg_32b(reinterpret_cast<const double *>(rpos + 2 * (size_t)k), pk);
-        double dxd = __dsub_rn(xi, pk[0]), dyd = __dsub_rn(yi, pk[1]), dzd = __dsub_rn(zi, pk[2]);
-        const double r2d = pair_image(dxd, dyd, dzd, bx, nbr_sh, ent, -1.0);
-        tk = (int)__double_as_longlong(pk[3]);
-        const R irv = vrad[ti * ntypes + tk];
-        if (r2d <= vf.off2 && irv > R(0.0)) {
-          const unsigned code = pair_primary(nbr_sh, ent) ? vexcl_code(i, k, eptr, ek, ecode, elo, ehi) : 0u;
-          mask = c_vscales.v[(code >> 7) & 3u];
-          pass = mask > R(0.0);
-          dx = (R)dxd; dy = (R)dyd; dz = (R)dzd; r2 = (R)r2d;
-          qflags = (r2d > vf.cut2 ? 1 : 0) | (pair_counted(i, k, nbr_sh, ent) ? 2 : 0);
-        }
-      }
-      const unsigned bal = __ballot_sync(0xffffffffu, pass);
-      if (pass) {
-        const int q = qn + __popc(bal & ((1u << lane) - 1u));
-        qk[q] = k; qt[q] = tk; qf[q] = qflags; qx[q] = dx; qy[q] = dy; qz[q] = dz; qr[q] = r2; qm[q] = mask;
-      }
-      qn += __popc(bal);
-      __syncwarp();
-      if (qn >= 32) {
-        pair_math(qk[lane], qt[lane], qf[lane], qx[lane], qy[lane], qz[lane], qr[lane], qm[lane]);
-        __syncwarp();
-        if (lane < qn - 32) {
-          const int q = lane + 32;
-          qk[lane] = qk[q]; qt[lane] = qt[q]; qf[lane] = qf[q]; qx[lane] = qx[q]; qy[lane] = qy[q];
-          qz[lane] = qz[q]; qr[lane] = qr[q]; qm[lane] = qm[q];
-        }
-        __syncwarp();
+    for (int base = 0; base < m; base += 32 * kScan) {
+      qn += scan_row(row, base, m, fi, irpos, nbr_sh, bx, bound, queue, head + qn);
+      while (qn >= 32) {
+        pair_math();
+        head += 32;
         qn -= 32;
       }
+      __syncwarp();
     }
-    if (lane < qn) pair_math(qk[lane], qt[lane], qf[lane], qx[lane], qy[lane], qz[lane], qr[lane], qm[lane]);
+    if (lane < qn) pair_math();
+    __syncwarp();
     e = warp_sum(e);
     const double Gx = warp_sum((double)gx), Gy = warp_sum((double)gy), Gz = warp_sum((double)gz);
   #pragma unroll
@@ -251,16 +236,19 @@ __device__ __forceinline__ void k_vdw_distribute(VGrid vg, int n, const double *
 
 
 // One vdW launch.  The batch instance is held to four resident blocks of 256 threads in
-// the FP32 form (64 registers, as the single-system instance uses).
+// the FP32 form (64 registers).  The FP64 instance is held to three (80 registers), so that
+// a block of it and a plane of the FP64 transforms (up to 168 registers, 256 threads) fit
+// one SM: the solver's transforms run beside it.
 template <typename R, bool ALCH>
 static void vdw_launch(Handle &h, bool grad, cudaStream_t st, const VdwForm &vf, int blocks) {
-  launch_on<k_vdw<R, ALCH>, 256, 0, sizeof(R) == 4 ? 4 : 0>(
-      h.rec, blocks, 256, 0, st, h.n, (const double *)h.d_rx, (const double *)h.d_ry, (const double *)h.d_rz, h.box,
+  launch_split_on<k_vdw<R, ALCH>, 256, sizeof(R) == 8 && !ALCH ? 3 : 0, sizeof(R) == 4 ? 4 : 0>(
+      h.rec, h.carve, blocks, 256, 0, st, h.n, (const double *)h.d_rx, (const double *)h.d_ry, (const double *)h.d_rz, h.box,
       (const int *)h.d_vtype, h.ntypes, (const double *)h.d_vrad, (const double *)h.d_veps, (const int *)h.d_nbr,
       (const int *)h.d_nbr_cnt, h.cap_nbr, (const int *)h.d_nbr_sh, (const int *)h.d_excl_ptr,
       (const int *)h.d_excl_k, (const unsigned *)h.d_excl_code, (const int *)h.d_excl_lo, (const int *)h.d_excl_hi,
       vf, h.scales, grad ? 1 : 0, h.d_eatom, h.d_catom, h.d_gred, (const int *)h.d_soft, (const int *)h.d_mol, h.alch,
-      h.d_eatom + 7 * (size_t)h.n, h.d_eatom + 8 * (size_t)h.n, h.d_lgred, (const double2 *)h.d_rpos);
+      h.d_eatom + 7 * (size_t)h.n, h.d_eatom + 8 * (size_t)h.n, h.d_lgred, (const double2 *)h.d_rpos,
+      (const int4 *)h.d_irpos);
 }
 
 void launch_vdw(Handle &h, bool grad, cudaStream_t st) {
@@ -282,13 +270,11 @@ void launch_vdw(Handle &h, bool grad, cudaStream_t st) {
   vf.c5 = -6.0 / den;
   vf.cut = cut;
   vf.iwidth = 1.0 / (off - cut);
-  // In a captured evaluation vdW is a low-priority branch beside the permanent field and
-  // the solver: one block of eight warps per SM, warps striding over atoms.  Its blocks
-  // stay resident until the term is done, so a wider branch holds the registers the
-  // other kernels need: at four blocks per SM (the whole register file) the permanent
-  // field and reciprocal chain waited ~140 us for it on the 24k box; at one block per SM
-  // it runs in the solver's idle issue slots (657-668 -> 696 evals/s; 128-thread blocks
-  // or two per SM measured slower).
+  // In a captured evaluation vdW is a low-priority branch beside the solver: one block of
+  // eight warps per SM, warps striding over atoms.  Its blocks stay resident until the term
+  // is done, so a wider branch holds the registers the other kernels need (at four blocks
+  // per SM, the whole register file, they waited for it); at one it runs in the solver's
+  // idle issue slots.
   const int full = nblocks((int64_t)h.n * 32, 256);
   const int blocks = h.capturing ? std::min(full, h.num_sms) : full;
   if (h.alch.active) {
