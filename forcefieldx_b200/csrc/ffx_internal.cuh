@@ -211,7 +211,7 @@ __device__ __forceinline__ float fixed_r2(const int4 &a, const int4 &b, const Bo
 
 // A row scan tests r^2 <= cutoff^2 on the fixed-point fractions first, against a bound this
 // much larger; what passes is tested exactly, in FP64, where it is worked on.
-__device__ __forceinline__ float scan_bound(double off2) { return (float)(off2 * 1.0001); }
+__host__ __device__ __forceinline__ float scan_bound(double off2) { return (float)(off2 * 1.0001); }
 
 // Entries that pass a row scan, queued by the scanning warp and worked on 32 at a time: a
 // ring of kQueue (partner, place in the row), so that what stays behind after 32 need not
@@ -589,6 +589,7 @@ struct Handle {
   // dipoles of the PCG fields, [n][8] of double (plain) or float (mixed): d_recF holds
   // the dipoles whose field is taken (u, then p), d_recP holds alpha r.
   double2 *d_pos = nullptr;
+  int4 *d_cell_fixed = nullptr;                 // [n] irpos in cell order, w the atom
   int4 *d_ipos = nullptr, *d_irpos = nullptr;   // fixed-point fractions of x and of the reduced r
   void *d_recF = nullptr, *d_recP = nullptr;
   void *d_erec = nullptr;                     // [n][kRecStride] real-space gather records
