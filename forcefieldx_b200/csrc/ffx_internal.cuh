@@ -468,6 +468,17 @@ struct PcgState {
   int pad;
 };
 
+// Where an evaluation's last kernel puts what the host reads (pinned host memory; terms
+// null: nowhere).
+struct HostResults {
+  double *terms;
+  long long *counts;
+  int *flags;
+  PcgState *pcg;
+  const int *d_flags;
+  const PcgState *d_pcg;
+};
+
 // vdW softcore constants of the current lambda (VanDerWaals.setLambda).
 struct AlchConst {
   double sc1, dsc1dL, d2sc1dL2, sc2, dsc2dL, d2sc2dL2;
@@ -623,6 +634,7 @@ struct Handle {
   int carve = 28;                             // shared-memory split of the kernels that run beside the mesh passes
 
   // ---- outputs
+  double *d_param = nullptr, *h_param = nullptr;   // parameter gradients: workspace, pinned results
   double *d_grad = nullptr, *d_torque = nullptr;  // [3][n]
   double *d_gred = nullptr;                        // [3][n] vdW reduced-site force
   double *d_eatom = nullptr;                       // [kEnergyRows][n] per-atom energy terms
@@ -752,8 +764,9 @@ void launch_elec_restore(Handle &h);
 void launch_lambda_grad_add(Handle &h, double *out);
 void launch_zero_soft_multipoles(Handle &h);
 void launch_assemble(Handle &h, double *d_grad_xyz);
-void launch_reduce_results(Handle &h);
-int param_gradients(Handle &h, double *dEdM, double *dEdA);
+void launch_sums(Handle &h);
+void launch_results(Handle &h, bool solver);
+int param_gradients(Handle &h, double *scratch, double *dEdM, double *dEdA);
 int setup_pme(Handle &h);   // FFXG_OK or a status (h.err set)
 
 inline int nblocks(int64_t n, int t) { return (int)((n + t - 1) / t); }

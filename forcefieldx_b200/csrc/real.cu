@@ -1005,10 +1005,8 @@ __global__ void k_param_finish(int n, const double *__restrict__ phi, const doub
 }
 
 // dE/dM [n][10] (device) and dE/dalpha [n] (device) of the last evaluation's state.
-int param_gradients(Handle &h, double *d_dM, double *d_dA) {
+int param_gradients(Handle &h, double *scratch, double *d_dM, double *d_dA) {
   const size_t N = h.n;
-  double *scratch = nullptr;
-  if (cudaMallocAsync(&scratch, 10 * N * sizeof(double), h.stream) != cudaSuccess) return FFXG_ERR_CUDA;
   const bool pol = h.prm.polarization != FFXG_POLAR_NONE;
   k_param_real<<<nblocks((int64_t)h.n * 32, 128), 128, 0, h.stream>>>(
       h.n, h.d_x, h.d_y, h.d_z, h.box, h.d_gm, h.d_uD, h.d_uP, h.d_ipdamp, h.d_thole, h.d_ewl, h.d_ewl_cnt,
@@ -1026,7 +1024,6 @@ int param_gradients(Handle &h, double *d_dM, double *d_dA) {
   pc.pol = pol ? 1 : 0;
   k_param_finish<<<nblocks(h.n, 128), 128, 0, h.stream>>>(h.n, scratch, h.d_gm, h.d_cphi, h.d_cphiI, h.d_cphiP,
                                                           h.d_uD, h.d_uP, h.d_polar, h.d_rot, pc, d_dM, d_dA);
-  cudaFreeAsync(scratch, h.stream);
   h.launches += 2;
   return cudaGetLastError() == cudaSuccess ? FFXG_OK : FFXG_ERR_CUDA;
 }

@@ -357,23 +357,36 @@ __device__ __forceinline__ void k_sum_partial(VGrid vg, int n, const double *__r
 }
 
 // Row t of the totals by warp t: lane l sums blocks l, l + 32, ..., then a fixed shuffle
-// tree (the same order on every call).
+// tree (the same order on every call).  The evaluation's last kernel: with host.terms set it
+// also writes everything the host reads (totals, counts, flags, solver state) to the pinned
+// buffers, so that no copies of a few bytes follow it (four of them, one after another, took
+// 25 us).
 __device__ __forceinline__ void k_sum_final(VGrid vg, int nb, const double *__restrict__ pe, const long long *__restrict__ pc, double *out,
-                            long long *cout) {
+                            long long *cout, const HostResults &host) {
   const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+  if (host.terms && threadIdx.x == 0) {
+    *host.flags = *host.d_flags;
+    if (host.pcg) *host.pcg = *host.d_pcg;
+  }
   if (row < kNE) {
     double s = 0.0;
     for (int b = lane; b < nb; b += 32) s += pe[b * kNE + row];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) out[row] = s;
+    if (lane == 0) {
+      out[row] = s;
+      if (host.terms) host.terms[row] = s;
+    }
   } else if (row < kNE + kNC) {
     const int t = row - kNE;
     long long s = 0;
     for (int b = lane; b < nb; b += 32) s += pc[b * kNC + t];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) cout[t] = s;
+    if (lane == 0) {
+      cout[t] = s;
+      if (host.terms) host.counts[t] = s;
+    }
   }
 }
 
@@ -494,15 +507,31 @@ void launch_zero_soft_multipoles(Handle &h) {
   FFX_LAUNCHED(h);
 }
 
-void launch_reduce_results(Handle &h) {
-  double *pe = h.d_partials;
-  long long *pc = reinterpret_cast<long long *>(h.d_partials + kSumBlocks * kNE);
-  const int nb = std::min(kSumBlocks, std::max(1, (h.n + 255) / 256));   // fewer blocks for small systems
-  launch_on<k_sum_partial, 0, 0>(h.rec, nb, 256, 0, h.stream, h.n, (const double *)h.d_eatom,
-                                 (const long long *)h.d_catom, pe, pc);
-  launch_on<k_sum_final, 0, 0>(h.rec, 1, 32 * (kNE + kNC), 0, h.stream, nb, (const double *)pe,
-                               (const long long *)pc, h.d_result, h.d_cresult);
-  h.launches += 2;
+static int sum_blocks(const Handle &h) {   // fewer blocks for small systems
+  return std::min(kSumBlocks, std::max(1, (h.n + 255) / 256));
+}
+
+// The energy and count sums in two launches: launch_sums (which reads only the per-atom
+// rows) and, when flags and solver state are final, launch_results.
+void launch_sums(Handle &h) {
+  launch_on<k_sum_partial, 0, 0>(h.rec, sum_blocks(h), 256, 0, h.stream, h.n, (const double *)h.d_eatom,
+                                 (const long long *)h.d_catom, h.d_partials,
+                                 reinterpret_cast<long long *>(h.d_partials + kSumBlocks * kNE));
+  FFX_LAUNCHED(h);
+}
+
+void launch_results(Handle &h, bool solver) {
+  HostResults host{};
+  if (!h.rec) {
+    host.terms = h.h_scalars;
+    host.counts = reinterpret_cast<long long *>(h.h_flags + 2);
+    host.flags = h.h_flags;
+    host.d_flags = h.d_flags;
+    if (solver) { host.pcg = h.h_pcg; host.d_pcg = h.d_pcg; }
+  }
+  launch_on<k_sum_final, 0, 0>(h.rec, 1, 32 * (kNE + kNC), 0, h.stream, sum_blocks(h), (const double *)h.d_partials,
+                               (const long long *)(h.d_partials + kSumBlocks * kNE), h.d_result, h.d_cresult, host);
+  FFX_LAUNCHED(h);
 }
 
 }  // namespace ffx
