@@ -221,6 +221,13 @@ struct PairQueue {
   int2 e[kQueue];
 };
 
+// A list entry read once: past the L1, which is left to the gathered records.
+__device__ __forceinline__ int ld_stream(const int *p) {
+  int k;
+  asm("ld.global.nc.L1::no_allocate.s32 %0, [%1];" : "=r"(k) : "l"(__cvta_generic_to_global(p)));
+  return k;
+}
+
 // One step of a row scan by a warp: entries base .. base + 32 kScan - 1 of the row's m, the
 // loads of every chunk in flight together (a chunk at a time, the two dependent gathers are
 // most of a scan's time: vdW 158 us, against 137 with four).  The FP32 test costs a third of
@@ -236,7 +243,7 @@ __device__ __forceinline__ int scan_row(const int *__restrict__ row, int base, i
 #pragma unroll
   for (int u = 0; u < kScan; u++) {
     const int a = base + 32 * u + lane;
-    k[u] = a < m ? row[a] : -1;
+    k[u] = a < m ? ld_stream(row + a) : -1;
   }
   if (!sh) {
 #pragma unroll
@@ -389,15 +396,30 @@ __device__ __forceinline__ void store_pair(PairRec<double> *p, size_t e, double 
 __device__ __forceinline__ void store_pair(PairRec<float> *p, size_t e, float x, float y, float z, float a) {
   p[e].v = make_float4(x, y, z, a);
 }
+// A cached pair is read once by each field: past the L1, which is left to the gathered
+// source records (24,000 atoms mixed: pair field 268 -> 245 us an evaluation, the whole 1,240
+// -> 1,170; 9,738 FP64 1,095 -> 1,020), and with ONCE first to be evicted from L2.  The FP64
+// field's rows (137 MB on the 24,000-atom box) take ONCE: they would displace the mesh and
+// the solver's vectors (1,783 -> 1,717 us); the preconditioner's rows, and the FP32 field's
+// (1,175 against 1,178 us, and 3,373 against 3,420 at 81,000 atoms), gain from what L2 keeps.
+template <bool ONCE>
 __device__ __forceinline__ void load_pair(const PairRec<double> *__restrict__ p, size_t e, double &x, double &y,
                                           double &z, double &a) {
-  const double2 u = __ldg(&p[e].xy), v = __ldg(&p[e].za);
-  x = u.x; y = u.y; z = v.x; a = v.y;
+  if constexpr (ONCE)
+    asm("ld.global.nc.L1::no_allocate.L2::evict_first.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(x), "=d"(y), "=d"(z), "=d"(a)
+        : "l"(__cvta_generic_to_global(p + e)));
+  else
+    asm("ld.global.nc.L1::no_allocate.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(x), "=d"(y), "=d"(z), "=d"(a)
+        : "l"(__cvta_generic_to_global(p + e)));
 }
+template <bool ONCE>
 __device__ __forceinline__ void load_pair(const PairRec<float> *__restrict__ p, size_t e, float &x, float &y,
                                           float &z, float &a) {
-  const float4 u = __ldg(&p[e].v);
-  x = u.x; y = u.y; z = u.z; a = u.w;
+  asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+      : "=f"(x), "=f"(y), "=f"(z), "=f"(a)
+      : "l"(__cvta_generic_to_global(p + e)));
 }
 
 // The dyadic coefficient B of cached pair e and its partner k.  Plain form: B in its own
@@ -409,12 +431,13 @@ __device__ __forceinline__ void store_pair_b(float *pb, size_t e, int k, float b
 }
 __device__ __forceinline__ void load_pair_b(const double *__restrict__ pb, const int *__restrict__ lst, size_t e,
                                             int &k, double &b) {
-  k = __ldg(lst + e);
-  b = __ldg(pb + e);
+  k = ld_stream(lst + e);
+  asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(b) : "l"(__cvta_generic_to_global(pb + e)));
 }
 __device__ __forceinline__ void load_pair_b(const float *__restrict__ pb, const int *__restrict__, size_t e, int &k,
                                             float &b) {
-  const int2 t = __ldg(reinterpret_cast<const int2 *>(pb) + e);
+  int2 t;
+  asm("ld.global.nc.L1::no_allocate.v2.s32 {%0, %1}, [%2];" : "=r"(t.x), "=r"(t.y) : "l"(__cvta_generic_to_global(reinterpret_cast<const int2 *>(pb) + e)));
   k = t.x;
   b = __int_as_float(t.y);
 }

@@ -189,7 +189,7 @@ __device__ __forceinline__ void pair_field(int i, int sub, const int *__restrict
     }
 #pragma unroll
     for (int u = 0; u < NU; u++) {
-      load_pair(pr, e0 + ix[u], xx[u], yy[u], zz[u], AA[u]);
+      load_pair<sizeof(T) == 8 && G == kEwaldGroup>(pr, e0 + ix[u], xx[u], yy[u], zz[u], AA[u]);
       get_rec(rec, kk[u], ss[u]);
     }
 #pragma unroll
