@@ -436,17 +436,40 @@ __device__ __forceinline__ void k_fft_axis(VGrid vg, typename Vec2<S>::type *gri
   const int gi = vg.bid % ax.groups_inner, go = vg.bid / ax.groups_inner;
   const size_t base = (size_t)gi * ax.group_step_inner + (size_t)go * ax.group_step_outer;
   const bool contiguous = (ax.stride == 1);
-  for (int t = threadIdx.x; t < len * L; t += blockDim.x) {
-    const int l = contiguous ? t / len : t % L, j = contiguous ? t % len : t / L;
-    const size_t g = base + (size_t)l * ax.line_step + (size_t)j * ax.stride;
-    if (FROMD) {
-      const double2 q = make_double2(src[g], src[src_ng + g]);
-      if (sizeof(S) == 4 && (quant_out(q.x) || quant_out(q.y))) atomicOr(flags, FLAG_QUANT_RANGE);
-      src[g] = 0.0;
-      src[src_ng + g] = 0.0;
-      buf0[j * L + l] = mk2<S>((S)q.x, (S)q.y);
-    } else {
-      buf0[j * L + l] = grid[g];
+  if constexpr (FROMD) {
+    // Several items' loads go out before the first of them is cleared: a load may not pass a
+    // store to the same mesh, so that one item at a time each waits for the memory's round
+    // trip (128^3 FP64: 165 us a launch, 53 with eight; FP32 would lose a resident block to
+    // the registers of eight).
+    constexpr int U = sizeof(S) == 8 ? 8 : 4;
+    for (int t0 = threadIdx.x; t0 < len * L; t0 += U * blockDim.x) {
+      double re[U], im[U];
+      size_t g[U];
+      int at[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int t = t0 + u * blockDim.x;
+        const int l = contiguous ? t / len : t % L, j = contiguous ? t % len : t / L;
+        g[u] = base + (size_t)l * ax.line_step + (size_t)j * ax.stride;
+        at[u] = j * L + l;
+        if (t < len * L) {
+          re[u] = src[g[u]];
+          im[u] = src[src_ng + g[u]];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (t0 + u * (int)blockDim.x >= len * L) break;
+        if (sizeof(S) == 4 && (quant_out(re[u]) || quant_out(im[u]))) atomicOr(flags, FLAG_QUANT_RANGE);
+        src[g[u]] = 0.0;
+        src[src_ng + g[u]] = 0.0;
+        buf0[at[u]] = mk2<S>((S)re[u], (S)im[u]);
+      }
+    }
+  } else {
+    for (int t = threadIdx.x; t < len * L; t += blockDim.x) {
+      const int l = contiguous ? t / len : t % L, j = contiguous ? t % len : t / L;
+      buf0[j * L + l] = grid[base + (size_t)l * ax.line_step + (size_t)j * ax.stride];
     }
   }
   __syncthreads();
