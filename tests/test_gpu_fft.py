@@ -23,6 +23,7 @@ MESHES = [
     (64, 64, 64), (96, 80, 72), (120, 128, 10),    # one chunk, several chunks, factor 16
     (160, 160, 6),                                 # a plane beyond one CTA: per-axis passes
     (11, 20, 24), (20, 13, 16), (16, 18, 17),      # a general prime along each axis
+    (64, 16, 11), (16, 64, 13), (16, 11, 64),      # per-axis passes of length 64, each kind
 ]
 
 

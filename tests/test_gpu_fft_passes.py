@@ -60,3 +60,13 @@ def test_first_pass_keeps_its_loads_in_flight():
     behind the store that clears the item before it, the ratio was 2.6 to 3.5.)"""
     x0, _, _, _, x1 = _passes((128, 128, 128), 0)
     assert x0 < 2.0 * x1, (x0, x1)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_length_64_passes_without_run_time_divisions(precision):
+    """A 48 x 64 x 77 mesh, 16 lines a block along x and y: the y pass (length 64, radix 4
+    three times) has as many points and stages as the x pass (length 48, radices 4, 4 and 3),
+    and its indices need no run-time division, half of the x pass: the bar is 0.65 of its
+    time."""
+    _, _, _, y, x = _passes((48, 64, 77), precision)
+    assert y < 0.65 * x, (x, y)
