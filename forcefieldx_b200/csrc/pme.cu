@@ -761,10 +761,14 @@ template <typename S, bool INV, bool WIDE>
 struct FftPlanePass {
   using V = typename Vec2<S>::type;
   static constexpr int T = fft_plane_threads<S, WIDE>(), B = fft_plane_blocks<S, WIDE>();
+  // Dynamic shared memory a block may have: the batch instance stages its arguments too.
+  static constexpr size_t max_smem() {
+    return 227 * 1024 - (sizeof(Pack<V *, FftPlan, const V *, int, double *, size_t, int *>) + 15) / 16 * 16;
+  }
   static void launch(Handle &h, int block, size_t smem, V *mesh, const FftPlan &pl, const V *tw, int tw_step,
                      double *src, size_t ng) {
-    launch_split_on<k_fft_plane<S, INV, WIDE>, T, B>(h.rec, h.carve, pl.line[2].n, block, smem, h.stream, mesh, pl, tw, tw_step, src,
-                                               ng, h.d_flags);
+    launch_split_on<k_fft_plane<S, INV, WIDE>, T, B>(h.rec, h.carve, pl.line[2].n, block, smem, h.stream, mesh, pl,
+                                                     tw, tw_step, src, ng, h.d_flags);
   }
   static cudaError_t raise(int need) {
     const cudaError_t e1 =
@@ -781,7 +785,8 @@ struct FftZPass {
   using V = typename Vec2<S>::type;
   static void launch(Handle &h, int blocks, int block, size_t smem, V *mesh, const FftPlan &pl, const V *tw,
                      int tw_step, const S *G) {
-    launch_split_on<k_fft_z<S, WIDE>, 256, 0>(h.rec, h.carve, blocks, block, smem, h.stream, mesh, pl, tw, tw_step, G);
+    launch_split_on<k_fft_z<S, WIDE>, 256, 0>(h.rec, h.carve, blocks, block, smem, h.stream, mesh, pl, tw, tw_step,
+                                              G);
   }
   static cudaError_t raise(int need) {
     const cudaError_t e1 = cudaFuncSetAttribute(one_fn<k_fft_z<S, WIDE>, 256, 0, V *, FftPlan, const V *, int, const S *>(),
@@ -852,7 +857,7 @@ static bool plan_fft(const int nf[3], size_t value, FftPlan &p) {
   p = FftPlan{};
   for (int d = 0; d < 3; d++)
     if (!fft_line(nf[d], p.line[d])) return false;
-  constexpr size_t kMax = 227 * 1024;
+  constexpr size_t kMax = FftPlanePass<double, false, false>::max_smem();
   size_t limit = 100 * 1024;
   for (int parts = 1; parts <= 16; parts++) {
     p.row_chunk = (nf[1] + parts - 1) / parts;

@@ -185,3 +185,27 @@ def test_large_batch_host_copies_and_nonfinite_coordinates():
         assert np.array_equal(e1, e0)
         for j in checked:
             _same(PRECISION_MIXED, b.terms[j], grads[j], hist[j], j)
+
+
+# One mesh of each form the convolution takes (csrc/pme.cu, plan_fft): narrow, wide in the
+# plane, wide along z only, one chunk and several, planes at the shared-memory limit beside
+# the batch instance's staged arguments, per-axis passes of general and of length-64 lines.
+MESHES = [(16, 20, 24), (27, 45, 16), (16, 18, 45), (40, 36, 32), (80, 72, 10), (256, 45, 6), (100, 240, 5),
+          (11, 20, 24), (24, 20, 13), (98, 16, 10), (64, 16, 11), (16, 11, 64)]
+
+
+@pytest.mark.parametrize("precision", [PRECISION_MIXED, PRECISION_FP64])
+def test_staged_batch_over_every_form_of_mesh(precision):
+    from forcefieldx_b200.system import small_water_box, water_params
+    w = []
+    for j, mesh in enumerate(MESHES):
+        s, edge = small_water_box(300 + 3 * j, seed=60 + j)
+        w.append((s, water_params(edge, pme_grid=mesh, precision=precision)))
+    systems, params = [s for s, _ in w], [p for _, p in w]
+    hist = [_single(s, p, [s.xyz, s.xyz])[1] for s, p in w]
+    with BatchEnergy(systems, params) as b:
+        for _ in range(2):
+            e, grads = b.energy_and_gradient([s.xyz for s in systems])
+            for j, mesh in enumerate(MESHES):
+                _same(precision, b.terms[j], grads[j], hist[j], mesh)
+        assert b.stages() > 50     # one launch per stage, not a branch per system
