@@ -848,26 +848,31 @@ static size_t fft_z_smem(const FftPlan &p, size_t value) { return (2 * (size_t)k
 
 // Whether the mesh takes the two-step passes: every axis has its two factors and a plane
 // fits one CTA's shared memory (FP32 up to about 150 x 150, FP64 100 x 100).  The first
-// axis goes in one chunk where that fits 100 KB, and else in as few as do (or as few as fit
-// at all): a chunk costs two barriers, a larger plane the L1 of the kernels beside it
-// (smem_split).  Device time of an evaluation with the limit at 160 / 120 / 100 / 60 KB:
-// 24,000 atoms FP64 2,042 / 1,787 / 1,799 / 1,899 us, 81,000 mixed 3,841 / 3,481 / 3,421 /
-// 3,553.
+// axis goes in as few chunks as bring the plane under 100 KB, if eight do: a chunk costs two
+// barriers, a larger plane the L1 of the kernels beside it (smem_split).  Device time of an
+// evaluation with that limit at 160 / 120 / 100 / 60 KB: 24,000 atoms FP64 2,042 / 1,787 /
+// 1,799 / 1,899 us, 81,000 mixed 3,841 / 3,481 / 3,421 / 3,553.  A plane that they do not
+// (its second axis' lines alone take that much) goes in as few as fit, three or more.  An
+// evaluation with at least 1 / 3 / 5 / 9 chunks there, 10,125 atoms: 80^3 FP64 1,332 / 1,294 /
+// 1,304 / 1,379 us, 96^3 FP64 1,460 / 1,468 / 1,478 / 1,598, 128^3 mixed 1,384 / 1,378 /
+// 1,408 / 1,496; a batch of twelve 3,000-atom boxes at 80^3 FP64 9,851 / 8,719 / 8,359 / 8,760.
 static bool plan_fft(const int nf[3], size_t value, FftPlan &p) {
   p = FftPlan{};
   for (int d = 0; d < 3; d++)
     if (!fft_line(nf[d], p.line[d])) return false;
   constexpr size_t kMax = FftPlanePass<double, false, false>::max_smem();
-  size_t limit = 100 * 1024;
-  for (int parts = 1; parts <= 16; parts++) {
-    p.row_chunk = (nf[1] + parts - 1) / parts;
-    p.col_chunk = (nf[0] + parts - 1) / parts;
-    p.by_row_chunk = fast_div(p.row_chunk);
-    p.by_col_chunk = fast_div(p.col_chunk);
-    if (fft_plane_smem(p, value) <= limit) return fft_z_smem(p, value) <= kMax;
-    if (parts == 8) limit = kMax;
-  }
-  return false;
+  auto fits = [&](int first, int last, size_t limit) {
+    for (int parts = first; parts <= last; parts++) {
+      p.row_chunk = (nf[1] + parts - 1) / parts;
+      p.col_chunk = (nf[0] + parts - 1) / parts;
+      if (fft_plane_smem(p, value) <= limit) return true;
+    }
+    return false;
+  };
+  if (!fits(1, 8, 100 * 1024) && !fits(3, 16, kMax)) return false;
+  p.by_row_chunk = fast_div(p.row_chunk);
+  p.by_col_chunk = fast_div(p.col_chunk);
+  return fft_z_smem(p, value) <= kMax;
 }
 
 // The shared-memory split (percent of the SM's 228 KB) under which a plane's CTA and a vdW

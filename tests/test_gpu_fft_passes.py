@@ -1,8 +1,9 @@
-"""Times of the per-axis mesh passes against each other.
+"""The mesh passes as they are launched, from the activity trace.
 
 A mesh that does not take the two-step passes goes through five passes, one axis each
 (csrc/pme.cu, k_fft_axis).  The bars compare passes of one run with one another, medians over
-its launches, so that neither the clock nor other work on the device decides them.
+its launches, so that neither the clock nor other work on the device decides them.  For the
+two-step passes the shared memory of a plane's block shows in how many chunks it is taken.
 """
 import json
 import os
@@ -37,20 +38,25 @@ with tempfile.NamedTemporaryFile(suffix=".json") as t:
     prof.export_chrome_trace(t.name)
     ev = [e for e in json.load(open(t.name))["traceEvents"] if e.get("cat") == "kernel"]
 ev.sort(key=lambda e: e["ts"])
-print(json.dumps([[e["name"], e["dur"]] for e in ev if "k_fft_axis" in e["name"]]))
+print(json.dumps([[e["name"], e["dur"], e["args"]["shared memory"]] for e in ev if "k_fft_" in e["name"]]))
 """
+
+
+def _trace(mesh, precision):
+    """(name, time in us, shared memory in bytes) of every transform launch of three evaluations."""
+    env = dict(os.environ, PYTHONPATH=ROOT)
+    out = subprocess.run([sys.executable, "-c", TRACE, json.dumps([mesh, precision])], env=env, cwd=ROOT, check=True,
+                         capture_output=True, text=True, timeout=300).stdout
+    return json.loads(out.strip().splitlines()[-1])
 
 
 def _passes(mesh, precision):
     """Median time (us) of each of a convolution's five passes: x, y, z, y, x."""
-    env = dict(os.environ, PYTHONPATH=ROOT)
-    out = subprocess.run([sys.executable, "-c", TRACE, json.dumps([mesh, precision])], env=env, cwd=ROOT, check=True,
-                         capture_output=True, text=True, timeout=300).stdout
-    ev = json.loads(out.strip().splitlines()[-1])
+    ev = _trace(mesh, precision)
     assert ev and len(ev) % 5 == 0
-    fused = [bool(re.search(r"k_fft_axis<(true|1)", n)) for n, _ in ev]
+    fused = [bool(re.search(r"k_fft_axis<(true|1)", n)) for n, _, _ in ev]
     assert fused == [False, False, True, False, False] * (len(ev) // 5)
-    return np.median(np.array([d for _, d in ev]).reshape(-1, 5), axis=0)
+    return np.median(np.array([d for _, d, _ in ev]).reshape(-1, 5), axis=0)
 
 
 def test_first_pass_keeps_its_loads_in_flight():
@@ -70,3 +76,18 @@ def test_length_64_passes_without_run_time_divisions(precision):
     time."""
     _, _, _, y, x = _passes((48, 64, 77), precision)
     assert y < 0.65 * x, (x, y)
+
+
+@pytest.mark.parametrize("n,f1,f2,precision,chunks", [
+    (32, 4, 8, 0, 1),        # the whole plane under 100 KB
+    (64, 8, 8, 0, 4),        # the fewest that bring it there
+    (80, 8, 10, 0, 3), (96, 8, 12, 0, 3),   # none of eight does: the fewest that fit, three or more
+    (100, 10, 10, 0, 4), (128, 8, 16, 1, 3)])
+def test_plane_goes_in_the_fewest_chunks(n, f1, f2, precision, chunks):
+    """n lines of f1 runs of f2 values at odd strides, of each chunk and of the whole plane,
+    and two twiddle tables."""
+    value = 8 if precision else 16
+    stride = f1 * (f2 | 1) | 1
+    want = ((-(-n // chunks) + n) * stride + 2 * n) * value
+    got = {sm for name, _, sm in _trace((n, n, 5), precision) if "k_fft_plane" in name}
+    assert got == {want}, (got, want)
