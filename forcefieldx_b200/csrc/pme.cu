@@ -725,13 +725,24 @@ static FftAxis make_axis(int axis, const int nf[3]) {
 }
 
 
-// The dynamic shared-memory limit of the generic FFT kernels is an attribute of each kernel
-// on a device, shared by every handle in the process.  It only ever grows: a handle raises
-// it to the largest line batch of its three axes, so a handle created later (with smaller
-// axes, or its largest axis in another position) never lowers a limit on which an earlier
-// handle's launches rely.
+// The dynamic shared-memory limit of an FFT kernel is an attribute of the kernel on a
+// device, shared by every handle in the process.  It only ever grows: a handle raises it, for
+// the passes its mesh takes, to what they need, so that a handle created later never lowers a
+// limit on which an earlier handle's launches rely.  Needs within the 48 KB that every kernel
+// has (less the batch instance's staged arguments) are left alone: setting an attribute loads
+// the kernel, 0.1 ms each in the process's first handle (every pass of both forms: 3 ms of
+// the 25 that creating it and its first evaluation take, 648 atoms FP64).
 static std::mutex g_fft_smem_mu;
-static std::map<int, int> g_fft_smem;   // device -> current attribute value (bytes)
+static std::map<std::pair<int, const void *>, int> g_fft_smem;   // (device, kernel) -> bytes
+static cudaError_t raise_smem(int device, const void *fn, int need) {
+  if (need <= 47 * 1024) return cudaSuccess;
+  std::lock_guard<std::mutex> lock(g_fft_smem_mu);
+  int &cur = g_fft_smem[{device, fn}];
+  if (need <= cur) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
+  if (e == cudaSuccess) cur = need;
+  return e;
+}
 
 // The generic FFT pass as launched by fft_convolution, with its argument types fixed so
 // that the instances whose shared-memory limit raise_fft_smem sets are the ones launched.
@@ -743,16 +754,13 @@ struct FftAxisPass {
     launch_on<k_fft_axis<FUSE, S, FROMD, LEN>, 256, 0>(h.rec, blocks, 256, smem, h.stream, grid, a, sign, tw, infl,
                                                        nfx, nfy, plane, ng, h.d_flags);
   }
-  static cudaError_t raise(int need) {
-    const cudaError_t e1 = cudaFuncSetAttribute(
-        one_fn<k_fft_axis<FUSE, S, FROMD, LEN>, 256, 0, V *, FftAxis, int, const V *, const S *, int, int, double *,
-               size_t, int *>(),
-        cudaFuncAttributeMaxDynamicSharedMemorySize, need);
-    const cudaError_t e2 = cudaFuncSetAttribute(
-        many_fn<k_fft_axis<FUSE, S, FROMD, LEN>, 256, 0, V *, FftAxis, int, const V *, const S *, int, int, double *,
-                size_t, int *>(),
-        cudaFuncAttributeMaxDynamicSharedMemorySize, need);
-    return e1 != cudaSuccess ? e1 : e2;
+  static cudaError_t raise(int device, size_t need) {
+    const cudaError_t e = raise_smem(device, one_fn<k_fft_axis<FUSE, S, FROMD, LEN>, 256, 0, V *, FftAxis, int, const V *,
+                                                    const S *, int, int, double *, size_t, int *>(), (int)need);
+    return e != cudaSuccess ? e
+                            : raise_smem(device, many_fn<k_fft_axis<FUSE, S, FROMD, LEN>, 256, 0, V *, FftAxis, int,
+                                                         const V *, const S *, int, int, double *, size_t, int *>(),
+                                         (int)need);
   }
 };
 
@@ -770,14 +778,12 @@ struct FftPlanePass {
     launch_split_on<k_fft_plane<S, INV, WIDE>, T, B>(h.rec, h.carve, pl.line[2].n, block, smem, h.stream, mesh, pl,
                                                      tw, tw_step, src, ng, h.d_flags);
   }
-  static cudaError_t raise(int need) {
-    const cudaError_t e1 =
-        cudaFuncSetAttribute(one_fn<k_fft_plane<S, INV, WIDE>, T, B, V *, FftPlan, const V *, int, double *, size_t, int *>(),
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, need);
-    const cudaError_t e2 =
-        cudaFuncSetAttribute(many_fn<k_fft_plane<S, INV, WIDE>, T, B, V *, FftPlan, const V *, int, double *, size_t, int *>(),
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, need);
-    return e1 != cudaSuccess ? e1 : e2;
+  static cudaError_t raise(int device, size_t need) {
+    const cudaError_t e = raise_smem(device, one_fn<k_fft_plane<S, INV, WIDE>, T, B, V *, FftPlan, const V *, int,
+                                                    double *, size_t, int *>(), (int)need);
+    return e != cudaSuccess ? e
+                            : raise_smem(device, many_fn<k_fft_plane<S, INV, WIDE>, T, B, V *, FftPlan, const V *, int,
+                                                         double *, size_t, int *>(), (int)need);
   }
 };
 template <typename S, bool WIDE>
@@ -788,37 +794,14 @@ struct FftZPass {
     launch_split_on<k_fft_z<S, WIDE>, 256, 0>(h.rec, h.carve, blocks, block, smem, h.stream, mesh, pl, tw, tw_step,
                                               G);
   }
-  static cudaError_t raise(int need) {
-    const cudaError_t e1 = cudaFuncSetAttribute(one_fn<k_fft_z<S, WIDE>, 256, 0, V *, FftPlan, const V *, int, const S *>(),
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize, need);
-    const cudaError_t e2 = cudaFuncSetAttribute(many_fn<k_fft_z<S, WIDE>, 256, 0, V *, FftPlan, const V *, int, const S *>(),
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize, need);
-    return e1 != cudaSuccess ? e1 : e2;
+  static cudaError_t raise(int device, size_t need) {
+    const cudaError_t e = raise_smem(device, one_fn<k_fft_z<S, WIDE>, 256, 0, V *, FftPlan, const V *, int, const S *>(),
+                                     (int)need);
+    return e != cudaSuccess ? e
+                            : raise_smem(device, many_fn<k_fft_z<S, WIDE>, 256, 0, V *, FftPlan, const V *, int,
+                                                         const S *>(), (int)need);
   }
 };
-
-template <typename S>
-static cudaError_t raise_fft_smem_of(int need) {
-  const cudaError_t e[9] = {FftAxisPass<false, S, false, 0>::raise(need), FftAxisPass<false, S, true, 0>::raise(need),
-                            FftAxisPass<true, S, false, 0>::raise(need), FftPlanePass<S, false, false>::raise(need),
-                            FftPlanePass<S, false, true>::raise(need), FftPlanePass<S, true, false>::raise(need),
-                            FftPlanePass<S, true, true>::raise(need),  FftZPass<S, false>::raise(need),
-                            FftZPass<S, true>::raise(need)};
-  for (cudaError_t q : e)
-    if (q != cudaSuccess) return q;
-  return cudaSuccess;
-}
-
-static cudaError_t raise_fft_smem(int device, int need) {
-  std::lock_guard<std::mutex> lock(g_fft_smem_mu);
-  int &cur = g_fft_smem[device];
-  if (need <= cur) return cudaSuccess;
-  const cudaError_t e[2] = {raise_fft_smem_of<double>(need), raise_fft_smem_of<float>(need)};
-  for (cudaError_t q : e)
-    if (q != cudaSuccess) return q;
-  cur = need;
-  return cudaSuccess;
-}
 
 static FastDiv fast_div(int n) { return {(unsigned)(((1ull << 32) + n - 1) / n), n}; }
 
@@ -844,6 +827,8 @@ static size_t fft_plane_smem(const FftPlan &p, size_t value) {
   const size_t RS = (size_t)(x.f1 * (x.f2 | 1)) | 1, CS = (size_t)(y.f1 * (y.f2 | 1)) | 1;
   return (std::max(p.row_chunk * RS + x.n * CS, y.n * RS + p.col_chunk * CS) + x.n + y.n) * value;
 }
+static bool fft_wide_plane(const FftPlan &p) { return p.line[0].f2 > 8 || p.line[1].f2 > 8; }
+static bool fft_wide_z(const FftPlan &p) { return p.line[2].f2 > 8; }
 static size_t fft_z_smem(const FftPlan &p, size_t value) { return (2 * (size_t)kFftZLines + 1) * p.line[2].n * value; }
 
 // Whether the mesh takes the two-step passes: every axis has its two factors and a plane
@@ -885,9 +870,36 @@ static int smem_split(size_t plane) {
   return 100;
 }
 
-// Dynamic shared memory of one generic FFT pass over axis a (both sizes of the mesh type
-// fit in the FP64 figure).
-static size_t fft_axis_smem(const FftAxis &a) { return 2 * (size_t)a.len * a.L * sizeof(double2); }
+// Dynamic shared memory of one per-axis pass: at most 4,096 values a block, twice.
+static size_t fft_axis_smem(const FftAxis &a, size_t value) { return 2 * (size_t)a.len * a.L * value; }
+
+// The limits of the passes that fft_convolution launches for the handle's mesh (an axis of
+// length 64 needs no more than 32 KB).
+template <typename S>
+static cudaError_t raise_fft_smem(const Handle &h) {
+  constexpr size_t value = 2 * sizeof(S);
+  cudaError_t e[3] = {};
+  if (h.fft_planned) {
+    const FftPlan &p = h.fft_plan;
+    const size_t plane = fft_plane_smem(p, value), z = fft_z_smem(p, value);
+    if (fft_wide_plane(p)) {
+      e[0] = FftPlanePass<S, false, true>::raise(h.device, plane);
+      e[1] = FftPlanePass<S, true, true>::raise(h.device, plane);
+    } else {
+      e[0] = FftPlanePass<S, false, false>::raise(h.device, plane);
+      e[1] = FftPlanePass<S, true, false>::raise(h.device, plane);
+    }
+    e[2] = fft_wide_z(p) ? FftZPass<S, true>::raise(h.device, z) : FftZPass<S, false>::raise(h.device, z);
+  } else {
+    const size_t x = fft_axis_smem(h.axes[0], value), y = fft_axis_smem(h.axes[1], value);
+    e[0] = FftAxisPass<false, S, true, 0>::raise(h.device, x);
+    e[1] = FftAxisPass<false, S, false, 0>::raise(h.device, std::max(x, y));
+    e[2] = FftAxisPass<true, S, false, 0>::raise(h.device, fft_axis_smem(h.axes[2], value));
+  }
+  for (cudaError_t q : e)
+    if (q != cudaSuccess) return q;
+  return cudaSuccess;
+}
 
 int setup_pme(Handle &h) {
   const int nfx = h.prm.pme_grid[0], nfy = h.prm.pme_grid[1], nfz = h.prm.pme_grid[2];
@@ -991,14 +1003,7 @@ int setup_pme(Handle &h) {
   const size_t value = h.mixed ? sizeof(float2) : sizeof(double2);
   h.fft_planned = plan_fft(nf, value, h.fft_plan);
   h.carve = smem_split(h.fft_planned ? fft_plane_smem(h.fft_plan, value) : 0);
-  size_t smem = 48 * 1024;
-  for (int d = 0; d < 3; d++) smem = std::max(smem, fft_axis_smem(h.axes[d]));
-  if (h.fft_planned) smem = std::max(smem, std::max(fft_plane_smem(h.fft_plan, value), fft_z_smem(h.fft_plan, value)));
-  if (smem > 227 * 1024) {
-    h.err = "PME grid dimension too long for the shared-memory FFT";
-    return FFXG_ERR_BAD_ARG;
-  }
-  const cudaError_t e = raise_fft_smem(h.device, (int)smem);
+  const cudaError_t e = h.mixed ? raise_fft_smem<float>(h) : raise_fft_smem<double>(h);
   if (e != cudaSuccess) {
     h.err = std::string("FFT shared-memory attribute: ") + cudaGetErrorString(e);
     return FFXG_ERR_CUDA;
@@ -1084,7 +1089,7 @@ static void fft_convolution(Handle &h, typename Vec2<S>::type *grid, const typen
   const int maxn = std::max(nfx, std::max(nfy, nfz));
   if (h.fft_planned) {
     const FftPlan &pl = h.fft_plan;
-    const bool wide = pl.line[0].f2 > 8 || pl.line[1].f2 > 8, wide_z = pl.line[2].f2 > 8;
+    const bool wide = fft_wide_plane(pl), wide_z = fft_wide_z(pl);
     if (wide) fft_planes<S, true>(h, pl, grid, twiddle, false);
     else fft_planes<S, false>(h, pl, grid, twiddle, false);
     const int blocks = (nfx * nfy + kFftZLines - 1) / kFftZLines;
@@ -1103,7 +1108,7 @@ static void fft_convolution(Handle &h, typename Vec2<S>::type *grid, const typen
     const FftAxis &a = h.axes[d];
     const int outer = (d == 0) ? nfz : ((d == 1) ? nfz : nfy);
     const int blocks = a.groups_inner * outer;
-    const size_t smem = 2 * (size_t)a.len * a.L * sizeof(V);
+    const size_t smem = fft_axis_smem(a, sizeof(V));
     const V *tw = twiddle + (size_t)d * maxn;
     const S *none = nullptr;
     auto pass = [&](auto len) {
@@ -1511,7 +1516,7 @@ extern "C" int ffxg_pme_recip_permanent_noalloc(const double *d_xyz, const doubl
     const int sign = (pass < 3) ? -1 : +1;
     const FftAxis ax = make_axis(d, nf);
     const int outer = (d == 2) ? nf[1] : nf[2];
-    const size_t smem = fft_axis_smem(ax);   // <= 32 KB at kNaMaxDim: no attribute needed
+    const size_t smem = fft_axis_smem(ax, sizeof(double2));   // <= 32 KB at kNaMaxDim: no attribute needed
     using OneFft = void (*)(double2 *, FftAxis, int, const double2 *, const double *, int, int, double *, size_t,
                             int *);
     const OneFft f =
