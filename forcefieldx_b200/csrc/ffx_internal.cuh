@@ -221,6 +221,20 @@ struct PairQueue {
   int2 e[kQueue];
 };
 
+// One 32-byte read-only global load: a single 256-bit access on sm_100 (one pass through
+// the L1 for a gathered record instead of two or three).  p must be 32-byte aligned and
+// point to global memory.
+__device__ __forceinline__ void ldg_32b(const float *p, float *v) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+      : "l"(__cvta_generic_to_global(p)));
+}
+__device__ __forceinline__ void ldg_32b(const double *p, double *v) {
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+      : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+      : "l"(__cvta_generic_to_global(p)));
+}
+
 // A list entry read once: past the L1, which is left to the gathered records.
 __device__ __forceinline__ int ld_stream(const int *p) {
   int k;
@@ -232,11 +246,11 @@ __device__ __forceinline__ int ld_stream(const int *p) {
 // loads of every chunk in flight together (a chunk at a time, the two dependent gathers are
 // most of a scan's time: vdW 158 us, against 137 with four).  The FP32 test costs a third of
 // the exact one's instructions, and nearly half of a buffered row fails it: vdW 195 -> 137 us
-// and the real-space field 154 -> 132 us on the 24,000-atom box, mixed form.  Appends what passes to the queue at `tail` and returns how many.
-// A multi-image row (sh set) lists shifts of the unwrapped coordinates: its entries all pass.
+// and the real-space field 154 -> 132 us on the 24,000-atom box, mixed form.  Appends what
+// passes to the queue at `tail` and returns how many.
 __device__ __forceinline__ int scan_row(const int *__restrict__ row, int base, int m, const int4 &fi,
-                                        const int4 *__restrict__ fixed, const int *sh, const Box &bx, float bound,
-                                        int2 *queue, int tail) {
+                                        const int4 *__restrict__ fixed, const Box &bx, float bound, int2 *queue,
+                                        int tail) {
   const int lane = threadIdx.x & 31;
   int k[kScan], count = 0;
   int4 f[kScan];
@@ -245,16 +259,43 @@ __device__ __forceinline__ int scan_row(const int *__restrict__ row, int base, i
     const int a = base + 32 * u + lane;
     k[u] = a < m ? ld_stream(row + a) : -1;
   }
-  if (!sh) {
 #pragma unroll
-    for (int u = 0; u < kScan; u++) f[u] = k[u] >= 0 ? __ldg(fixed + k[u]) : fi;
-  }
+  for (int u = 0; u < kScan; u++) f[u] = k[u] >= 0 ? __ldg(fixed + k[u]) : fi;
 #pragma unroll
   for (int u = 0; u < kScan; u++) {
-    const bool pass = k[u] >= 0 && (sh || fixed_r2(f[u], fi, bx) <= bound);
+    const bool pass = k[u] >= 0 && fixed_r2(f[u], fi, bx) <= bound;
     const unsigned bal = __ballot_sync(0xffffffffu, pass);
     if (pass)
       queue[(tail + count + __popc(bal & ((1u << lane) - 1u))) & (kQueue - 1)] = make_int2(k[u], base + 32 * u + lane);
+    count += __popc(bal);
+  }
+  __syncwarp();
+  return count;
+}
+
+// The same for a multi-image row, which lists images of the unwrapped coordinates `pos` by
+// the shifts `sh`: the shifted distance needs no wrap and is tested at once.  (With every
+// entry queued instead, the pair arithmetic ran on half-empty warps: field of a 128-system
+// batch of 96 to 580 atoms 958 us against 522 FP64, 458 against 315 mixed.)
+__device__ __forceinline__ int scan_row_images(const int *__restrict__ row, int base, int m,
+                                               const int *__restrict__ sh, double xi, double yi, double zi,
+                                               const double2 *__restrict__ pos, const Box &bx, double off2, int2 *queue,
+                                               int tail) {
+  const int lane = threadIdx.x & 31;
+  int count = 0;
+#pragma unroll 1
+  for (int a = base + lane; a < base + 32 * kScan + lane; a += 32) {
+    int k = 0;
+    bool pass = a < m;
+    if (pass) {
+      k = ld_stream(row + a);
+      double p[4];
+      ldg_32b(reinterpret_cast<const double *>(pos + 2 * (size_t)k), p);
+      double x = __dsub_rn(xi, p[0]), y = __dsub_rn(yi, p[1]), z = __dsub_rn(zi, p[2]);
+      pass = pair_image(x, y, z, bx, sh, a, -1.0) <= off2;
+    }
+    const unsigned bal = __ballot_sync(0xffffffffu, pass);
+    if (pass) queue[(tail + count + __popc(bal & ((1u << lane) - 1u))) & (kQueue - 1)] = make_int2(k, a);
     count += __popc(bal);
   }
   __syncwarp();
@@ -293,20 +334,6 @@ __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
-}
-
-// One 32-byte read-only global load: a single 256-bit access on sm_100 (one pass through
-// the L1 for a gathered record instead of two or three).  p must be 32-byte aligned and
-// point to global memory.
-__device__ __forceinline__ void ldg_32b(const float *p, float *v) {
-  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-      : "l"(__cvta_generic_to_global(p)));
-}
-__device__ __forceinline__ void ldg_32b(const double *p, double *v) {
-  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-      : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
-      : "l"(__cvta_generic_to_global(p)));
 }
 
 // Packed per-atom source records for the field gathers: T[8] per atom = (D xyz, CR xyz,

@@ -188,7 +188,8 @@ __device__ __forceinline__ void k_realspace_field(
   const float bound = scan_bound(off2);
   int qn = 0;
   for (int base = 0; base < cnt; base += 32 * kScan) {
-    qn += scan_row(row, base, cnt, fi, ipos, nbr_sh, bx, bound, queue, head + qn);
+    qn += nbr_sh ? scan_row_images(row, base, cnt, nbr_sh + (size_t)i * cap, xi, yi, zi, pos, bx, off2, queue, head + qn)
+                 : scan_row(row, base, cnt, fi, ipos, bx, bound, queue, head + qn);
     while (qn >= 32) {
       work(32);
       qn -= 32;

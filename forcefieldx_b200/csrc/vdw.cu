@@ -184,7 +184,9 @@ __device__ __forceinline__ void k_vdw(
         }
     };
     for (int base = 0; base < m; base += 32 * kScan) {
-      qn += scan_row(row, base, m, fi, irpos, nbr_sh, bx, bound, queue, head + qn);
+      qn += nbr_sh ? scan_row_images(row, base, m, nbr_sh + (size_t)i * cap, xi, yi, zi, rpos, bx, vf.off2, queue,
+                                     head + qn)
+                   : scan_row(row, base, m, fi, irpos, bx, bound, queue, head + qn);
       while (qn >= 32) {
         pair_math();
         head += 32;
