@@ -15,11 +15,14 @@
 
 namespace ffx {
 
-
+// The pair form's constants in the arithmetic's type, so that the kernel reads each where it
+// is used (from the parameter bank, or from a batch's staged arguments) and holds none.
+template <typename R>
 struct VdwForm {
-  double off2, cut2, t1n, gamma1, delta, gamma;
-  double c0, c1, c2, c3, c4, c5;
-  double cut, iwidth;   // taper start and 1 / (cutoff - taper start)
+  double off2, cut2;
+  R t1n, gamma1, delta, gamma;
+  R c0, c1, c2, c3, c4, c5;
+  R cut, iwidth;   // taper start and 1 / (cutoff - taper start)
 };
 
 __device__ __forceinline__ unsigned vexcl_code(int i, int k, const int *__restrict__ ptr, const int *__restrict__ ek,
@@ -39,7 +42,7 @@ __device__ __forceinline__ void k_vdw(
     const int *__restrict__ const &nbr, const int *__restrict__ const &nbr_cnt, int const &cap,
     const int *__restrict__ const &nbr_sh, const int *__restrict__ const &eptr,
     const int *__restrict__ const &ek, const unsigned *__restrict__ const &ecode,
-    const int *__restrict__ const &elo, const int *__restrict__ const &ehi, const VdwForm &vf,
+    const int *__restrict__ const &elo, const int *__restrict__ const &ehi, const VdwForm<R> &vf,
     const ScaleTables &c_vscales, int const &gradient, double * const &eatom, long long * const &catom,
     double * const &gred, const int *__restrict__ const &soft, const int *__restrict__ const &mol,
     const AlchConst &al, double * const &edl, double * const &ed2l, double * const &lgred,
@@ -51,9 +54,6 @@ __device__ __forceinline__ void k_vdw(
   for (int i = warp; i < n; i += nwarps) {
     const double xi = rx[i], yi = ry[i], zi = rz[i];
     const int ti = vtype[i];
-    const R delta = vf.delta, gamma = vf.gamma, gamma1 = vf.gamma1, t1n = vf.t1n;
-    const R c0 = vf.c0, c1 = vf.c1, c2 = vf.c2, c3 = vf.c3, c4 = vf.c4, c5 = vf.c5;
-    const R cut = vf.cut, iwidth = vf.iwidth;
     double e = 0.0, dl = 0.0, d2l = 0.0;
     R gx = 0, gy = 0, gz = 0, lx = 0, ly = 0, lz = 0;
     long long cnt = 0;
@@ -71,6 +71,8 @@ __device__ __forceinline__ void k_vdw(
     const float bound = scan_bound(vf.off2);
     int head = 0, qn = 0;
     auto pair_math = [&]() {
+      // A batch's staged arguments are read from here on, not held across the scan.
+      asm volatile("" ::: "memory");
       const int2 qw = queue[(head + lane) & (kQueue - 1)];
       const int k = qw.x;
       const size_t ent = (size_t)i * cap + qw.y;
@@ -112,13 +114,13 @@ __device__ __forceinline__ void k_vdw(
         const R rho2 = xmul(rho, rho);
         const R rhoDisp1 = xmul(xmul(rho2, rho2), rho2);
         const R rhoDisp = xmul(rhoDisp1, rho);
-        const R rd = xadd(rho, delta), rd2 = xmul(rd, rd);
+        const R rd = xadd(rho, vf.delta), rd2 = xmul(rd, rd);
         const R rhoDelta1 = xmul(xmul(rd2, rd2), rd2);
         const R rhoDelta = xmul(rhoDelta1, rd);
         const R t1d = R(1.0) / xadd(alpha, rhoDelta);
-        const R t2d = R(1.0) / xadd(xadd(alpha, rhoDisp), gamma);
-        const R t1 = xmul(t1n, t1d);
-        const R t2a = xmul(gamma1, t2d);
+        const R t2d = R(1.0) / xadd(xadd(alpha, rhoDisp), vf.gamma);
+        const R t1 = xmul(vf.t1n, t1d);
+        const R t2a = xmul(vf.gamma1, t2d);
         const R t2 = xadd(t2a, R(-2.0));
         const R eik = xmul(xmul(eps_lambda, t1), t2);
         R taper = R(1.0), dtaper = R(0.0);
@@ -126,15 +128,16 @@ __device__ __forceinline__ void k_vdw(
           if (sizeof(R) == 8) {
             // The polynomial summed left to right, as the reference sums its terms.
             const R r3 = xmul(r2, r), r4 = xmul(r2, r2), r5 = xmul(r2, r3);
-            taper = xadd(xfma(c1, r, xfma(c2, r2, xfma(c3, r3, xfma(c4, r4, xmul(c5, r5))))), c0);
-            dtaper = xadd(xfma(R(2.0) * c2, r, xfma(R(3.0) * c3, r2, xfma(R(4.0) * c4, r3, xmul(R(5.0) * c5, r4)))),
-                          c1);
+            taper = xadd(xfma(vf.c1, r, xfma(vf.c2, r2, xfma(vf.c3, r3, xfma(vf.c4, r4, xmul(vf.c5, r5))))), vf.c0);
+            dtaper = xadd(xfma(R(2.0) * vf.c2, r,
+                               xfma(R(3.0) * vf.c3, r2, xfma(R(4.0) * vf.c4, r3, xmul(R(5.0) * vf.c5, r4)))),
+                          vf.c1);
           } else {
             // The same quintic in t = (r - cut) / (off - cut): 1 - 10 t^3 + 15 t^4 - 6 t^5.
             // The power form above cancels ~1e6-sized terms and is unusable in FP32.
-            const R t = xmul(xadd(r, -cut), iwidth), t2 = xmul(t, t);
+            const R t = xmul(xadd(r, -vf.cut), vf.iwidth), t2 = xmul(t, t);
             taper = xfma(xmul(t2, t), xfma(t, xfma(R(-6), t, R(15)), R(-10)), R(1));
-            dtaper = xmul(xmul(t2, xfma(t, xfma(R(-30), t, R(60)), R(-30))), iwidth);
+            dtaper = xmul(xmul(t2, xfma(t, xfma(R(-30), t, R(60)), R(-30))), vf.iwidth);
           }
         }
         e += xmul(xmul(R(0.5), eik), taper);
@@ -237,14 +240,21 @@ __device__ __forceinline__ void k_vdw_distribute(VGrid vg, int n, const double *
 }
 
 
-// One vdW launch.  The batch instance is held to four resident blocks of 256 threads in
-// the FP32 form (64 registers).  The FP64 instance is held to three (80 registers), so that
-// a block of it and a plane of the FP64 transforms (up to 168 registers, 256 threads) fit
-// one SM: the solver's transforms run beside it.
+// One vdW launch.  The FP64 instance is held to three resident blocks of 256 threads (80
+// registers), so that a block of it and a plane of the FP64 transforms (up to 168 registers,
+// 256 threads) fit one SM: the solver's transforms run beside it.  A batch instance is held to
+// what it needs without spilling: three blocks in FP64 (80 registers), four in FP32 (64, with
+// 36 bytes spilled), one less each for the softcore pairs.  96 systems of 600 to 3,000 atoms,
+// three / two blocks FP64 1,040 / 1,375 us, four / three FP32 868 / 968; held across the scan,
+// the arguments took 138 registers, one block, in FP64 (2,407 us) and spilled 440 bytes a
+// thread in FP32 (1,483).
 template <typename R, bool ALCH>
-static void vdw_launch(Handle &h, bool grad, cudaStream_t st, const VdwForm &vf, int blocks) {
-  launch_split_on<k_vdw<R, ALCH>, 256, sizeof(R) == 8 && !ALCH ? 3 : 0, sizeof(R) == 4 ? 4 : 0>(
-      h.rec, h.carve, blocks, 256, 0, st, h.n, (const double *)h.d_rx, (const double *)h.d_ry, (const double *)h.d_rz, h.box,
+static void vdw_launch(Handle &h, bool grad, cudaStream_t st, const VdwForm<double> &d, int blocks) {
+  const VdwForm<R> vf = {d.off2, d.cut2, (R)d.t1n, (R)d.gamma1, (R)d.delta, (R)d.gamma, (R)d.c0, (R)d.c1, (R)d.c2,
+                         (R)d.c3, (R)d.c4, (R)d.c5, (R)d.cut, (R)d.iwidth};
+  launch_split_on<k_vdw<R, ALCH>, 256, sizeof(R) == 8 && !ALCH ? 3 : 0, (sizeof(R) == 4 ? 4 : 3) - (ALCH ? 1 : 0)>(
+      h.rec, h.carve, blocks, 256, 0, st, h.n, (const double *)h.d_rx, (const double *)h.d_ry, (const double *)h.d_rz,
+      h.box,
       (const int *)h.d_vtype, h.ntypes, (const double *)h.d_vrad, (const double *)h.d_veps, (const int *)h.d_nbr,
       (const int *)h.d_nbr_cnt, h.cap_nbr, (const int *)h.d_nbr_sh, (const int *)h.d_excl_ptr,
       (const int *)h.d_excl_k, (const unsigned *)h.d_excl_code, (const int *)h.d_excl_lo, (const int *)h.d_excl_hi,
@@ -255,7 +265,7 @@ static void vdw_launch(Handle &h, bool grad, cudaStream_t st, const VdwForm &vf,
 
 void launch_vdw(Handle &h, bool grad, cudaStream_t st) {
   if (h.vacuum) return;   // a vacuum sub-system carries electrostatics only
-  VdwForm vf{};
+  VdwForm<double> vf{};
   const double off = h.prm.vdw_cutoff, cut = h.prm.vdw_taper * h.prm.vdw_cutoff;
   vf.off2 = off * off;
   vf.cut2 = cut * cut;
