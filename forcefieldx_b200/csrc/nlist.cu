@@ -14,9 +14,12 @@
 
 namespace ffx {
 
+// Neighbouring cells reach kReach cells to each side (slabs are at least half the buffered
+// cutoff wide); all cells of an axis that has no more than that.
+constexpr int kReach = 2;
 struct CellOffsets {
   int n[3];
-  int off[3][5];
+  int off[2][2 * kReach + 1];   // along y and z; k_verlet takes an x row's cells in runs
 };
 
 // Interleaved [n][3] -> SoA and gather records, the reduced coordinates r = a*(x - x_p) + x_p
@@ -230,25 +233,26 @@ __device__ __forceinline__ void k_verlet(VGrid vg, int n, const double2 *__restr
       __syncwarp();
     }
   };
-  for (int oz = 0; oz < 5; oz++) {
-    const int dz = co.off[2][oz];
+  for (int oz = 0; oz < 2 * kReach + 1; oz++) {
+    const int dz = co.off[1][oz];
     if (dz == 0x7fff) break;
     const int z2 = ((cz + dz) % ncz + ncz) % ncz;
-    for (int oy = 0; oy < 5; oy++) {
-      const int dy = co.off[1][oy];
+    for (int oy = 0; oy < 2 * kReach + 1; oy++) {
+      const int dy = co.off[0][oy];
       if (dy == 0x7fff) break;
       const int y2 = ((cy + dy) % ncy + ncy) % ncy;
       const int first = (z2 * ncy + y2) * ncx;
-      if (ncx <= 5) {
+      const int lo = cx - kReach, hi = cx + kReach + 1;
+      if (ncx <= 2 * kReach + 1) {
         run(first, 0, ncx);
-      } else if (cx < 2) {
-        run(first, 0, cx + 3);
-        run(first, cx - 2 + ncx, ncx);
-      } else if (cx + 3 > ncx) {
-        run(first, 0, cx + 3 - ncx);
-        run(first, cx - 2, ncx);
+      } else if (lo < 0) {
+        run(first, 0, hi);
+        run(first, lo + ncx, ncx);
+      } else if (hi > ncx) {
+        run(first, 0, hi - ncx);
+        run(first, lo, ncx);
       } else {
-        run(first, cx - 2, cx + 3);
+        run(first, lo, hi);
       }
     }
   }
@@ -397,11 +401,13 @@ static CellOffsets cell_offsets(const int nc[3]) {
   CellOffsets co;
   for (int d = 0; d < 3; d++) {
     co.n[d] = nc[d];
-    for (int j = 0; j < 5; j++) co.off[d][j] = 0x7fff;
-    if (nc[d] >= 5) {
-      for (int j = 0; j < 5; j++) co.off[d][j] = j - 2;
+    if (d == 0) continue;
+    int *off = co.off[d - 1];
+    for (int j = 0; j < 2 * kReach + 1; j++) off[j] = 0x7fff;
+    if (nc[d] >= 2 * kReach + 1) {
+      for (int j = 0; j < 2 * kReach + 1; j++) off[j] = j - kReach;
     } else {
-      for (int j = 0; j < nc[d]; j++) co.off[d][j] = j;
+      for (int j = 0; j < nc[d]; j++) off[j] = j;
     }
   }
   return co;
