@@ -1,9 +1,9 @@
 """The mesh convolution's passes at the sizes where they change form.
 
-Meshes whose axes have two factors of at most 16 take the two-step passes (csrc/fft.cuh):
-the narrow instance up to factors of 8, the wide one above, a plane's first axis in one
-chunk or several (shared memory); a length with a prime factor above 7, or a plane beyond
-one CTA, takes the per-axis passes.  A 300-atom water box is evaluated on meshes of every
+Meshes whose axes have two factors among 1..10, 12, 15 and 16 take the two-step passes
+(csrc/fft.cuh): the narrow instance up to factors of 8, the wide one above, a plane's first
+axis in one chunk or several (shared memory).  A length without such factors (a prime above
+7, or a smooth one as 98, 125 or 162), or a plane beyond one CTA, takes the per-axis passes.  A 300-atom water box is evaluated on meshes of every
 form, odd and prime lengths among them, against the FP64 oracle: the plain form at the
 parity bar of test_gpu_parity (1e-8 relative per term, 1e-6 RMS gradient), the mixed form
 at its own (test_gpu_precision_mixed) and bit for bit on repeated calls.
@@ -24,6 +24,7 @@ MESHES = [
     (160, 160, 6),                                 # a plane beyond one CTA: per-axis passes
     (11, 20, 24), (20, 13, 16), (16, 18, 17),      # a general prime along each axis
     (64, 16, 11), (16, 64, 13), (16, 11, 64),      # per-axis passes of length 64, each kind
+    (125, 12, 8), (10, 98, 12), (12, 10, 162),     # smooth lengths without two factors
 ]
 
 

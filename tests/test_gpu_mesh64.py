@@ -1,9 +1,9 @@
 """64 x 64 x 64 meshes and the near list's fallback.
 
-1. FP64 form on a 64^3 mesh (the compile-time-length FFT passes) against the oracle at the
+1. FP64 form on a 64^3 mesh (each plane's x lines in four chunks) against the oracle at the
    parity bar: 1e-8 relative per term, 1e-6 gradient RMS, identical counts.
-2. Mixed form on the same mesh (X and Y passes fused by four-CTA clusters, the double
-   accumulation mesh cleared by its reader) at the mixed bar, bit for bit on repeated
+2. Mixed form on the same mesh (a plane in one chunk, the double accumulation mesh cleared by
+   its reader) at the mixed bar, bit for bit on repeated
    calls: a mesh left dirty by one call would change the next.
 3. A hydrogen whose vdW reduction factor is 0.5 (its reduced site half-way to the
    oxygen, 0.48 A from the atom): the offset exceeds the near list's 0.25 A margin, so
