@@ -1,4 +1,4 @@
-// fft.cuh -- mesh convolution of axes with two factors of at most 16.
+// fft.cuh -- mesh convolution of axes with two factors among 1..10, 12, 15 and 16.
 //
 // A length N = F1 F2 line is transformed in two steps, each a DFT held in registers:
 // step 1 takes the F1 elements j + r F2 (r < F1) of one j, step 2 the F2 results of one
@@ -9,7 +9,6 @@
 // the influence function and the inverse along z one (k_fft_z), the inverse of the planes
 // one (k_fft_plane<S, true>): three launches where the per-axis passes take five
 // (Complex3DParallel.convolution, N/fft/Complex3DParallel.java:445, 775-1010).
-//
 //
 // The meshes (0.06 to 14 MB) live in L2 and the launches are bound by latency: the round
 // trip to L2, three block barriers and the launch itself.  A whole plane per CTA, so that
@@ -31,8 +30,10 @@
 
 namespace ffx {
 
-// Threads of a plane's CTA, and resident blocks its registers are held to (the wide FP32
-// instance would spill at 64 registers).
+// Threads of a plane's CTA, and resident blocks its registers are held to: two of 512 threads
+// in FP32, 64 registers, at which the narrow forward instance spills 156 bytes (the planes are
+// read as FP64 values) and the wide instance would spill more, so that it has 384 threads and
+// no bound.
 template <typename S, bool WIDE> constexpr int fft_plane_threads() { return sizeof(S) == 8 ? 256 : WIDE ? 384 : 512; }
 template <typename S, bool WIDE> constexpr int fft_plane_blocks() { return sizeof(S) == 8 || WIDE ? 0 : 2; }
 constexpr int kFftZLines = 8;   // z lines per CTA: 64- or 128-byte runs of each z layer

@@ -9,7 +9,9 @@
 //   nbr[n][cap]      buffered Verlet list (both directions), nbr_cnt[n]
 //   ewl[n][capE]     real-space (Ewald) list, ewl_cnt[n]
 //   prl[n][capP]     preconditioner list, prl_cnt[n]
-//   grid[nz][ny][nx] interleaved complex PME mesh (double2)
+//   grid             PME accumulation mesh: real plane, then imaginary plane, each
+//                    [nz][ny][nx] (double); gridd / gridf the interleaved complex mesh of
+//                    the FP64 / mixed form
 #pragma once
 
 #include <cuda_runtime.h>
@@ -464,7 +466,9 @@ __device__ __forceinline__ void load_pair_b(const double *__restrict__ pb, const
 __device__ __forceinline__ void load_pair_b(const float *__restrict__ pb, const int *__restrict__, size_t e, int &k,
                                             float &b) {
   int2 t;
-  asm("ld.global.nc.L1::no_allocate.v2.s32 {%0, %1}, [%2];" : "=r"(t.x), "=r"(t.y) : "l"(__cvta_generic_to_global(reinterpret_cast<const int2 *>(pb) + e)));
+  asm("ld.global.nc.L1::no_allocate.v2.s32 {%0, %1}, [%2];"
+      : "=r"(t.x), "=r"(t.y)
+      : "l"(__cvta_generic_to_global(reinterpret_cast<const int2 *>(pb) + e)));
   k = t.x;
   b = __int_as_float(t.y);
 }

@@ -150,10 +150,6 @@ static int alloc_lists(Handle &h) {
 
 static int round32(double v) { return ((int)std::ceil(v) + 31) / 32 * 32; }
 
-// Crystal.updateCrystal (C/Crystal.java:1428-1548): lattice vectors as the rows of A^-1,
-// A their inverse (lower triangular: closed form), the volume and the perpendicular widths
-// 1 / |a*_d|, by the orthorhombic, monoclinic (only beta differs from 90) and general
-// branches.  Angles of 0 read as 90.
 // The lattice vectors over 2^32, the steps of the fixed-point fractions.
 static void set_steps(Box &b) {
   const double q = 1.0 / 4294967296.0;
@@ -161,6 +157,10 @@ static void set_steps(Box &b) {
   b.s11 = (float)(b.Ai11 * q); b.s21 = (float)(b.Ai21 * q); b.s22 = (float)(b.Ai22 * q);
 }
 
+// Crystal.updateCrystal (C/Crystal.java:1428-1548): lattice vectors as the rows of A^-1,
+// A their inverse (lower triangular: closed form), the volume and the perpendicular widths
+// 1 / |a*_d|, by the orthorhombic, monoclinic (only beta differs from 90) and general
+// branches.  Angles of 0 read as 90.
 static Box make_box(const double box[3], const double angles[3], double width[3]) {
   Box b{};
   b.a = box[0]; b.b = box[1]; b.c = box[2];

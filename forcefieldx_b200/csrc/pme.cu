@@ -805,8 +805,9 @@ struct FftZPass {
 
 static FastDiv fast_div(int n) { return {(unsigned)(((1ull << 32) + n - 1) / n), n}; }
 
-// n = f1 f2 with factors the register DFTs cover, the larger as small as it goes; false
-// when there is none (a prime factor above 7, or n beyond 256).
+// n = f1 f2 with factors the register DFTs cover, the larger as small as it goes; false when
+// there is none: a prime factor above 7, n beyond 256, or a smooth n without two such factors
+// (125, 162, 200, 216, 243, 250, and multiples of 7 from 98 on that take 14, 18, 20 or more).
 static bool fft_line(int n, FftLine &a) {
   static const int radix[] = {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 15, 16};
   a = FftLine{};
@@ -838,9 +839,9 @@ static size_t fft_z_smem(const FftPlan &p, size_t value) { return (2 * (size_t)k
 // evaluation with that limit at 160 / 120 / 100 / 60 KB: 24,000 atoms FP64 2,042 / 1,787 /
 // 1,799 / 1,899 us, 81,000 mixed 3,841 / 3,481 / 3,421 / 3,553.  A plane that they do not
 // (its second axis' lines alone take that much) goes in as few as fit, three or more.  An
-// evaluation with at least 1 / 3 / 5 / 9 chunks there, 10,125 atoms: 80^3 FP64 1,332 / 1,294 /
-// 1,304 / 1,379 us, 96^3 FP64 1,460 / 1,468 / 1,478 / 1,598, 128^3 mixed 1,384 / 1,378 /
-// 1,408 / 1,496; a batch of twelve 3,000-atom boxes at 80^3 FP64 9,851 / 8,719 / 8,359 / 8,760.
+// evaluation with at least 1 / 3 / 5 / 9 chunks there, 10,125 atoms: 80^3 FP64 1,221 / 1,232 /
+// 1,217 / 1,314 us, 96^3 FP64 1,361 / 1,360 / 1,380 / 1,516, 128^3 mixed 1,357 / 1,344 /
+// 1,378 / 1,426; a batch of twelve 3,000-atom boxes at 80^3 FP64 9,395 / 8,271 / 7,905 / 8,380.
 static bool plan_fft(const int nf[3], size_t value, FftPlan &p) {
   p = FftPlan{};
   for (int d = 0; d < 3; d++)
@@ -862,7 +863,8 @@ static bool plan_fft(const int nf[3], size_t value, FftPlan &p) {
 
 // The shared-memory split (percent of the SM's 228 KB) under which a plane's CTA and a vdW
 // block fit one SM: the smallest of the hardware's that does, since the rest is L1 for the
-// pair kernels' gathers.
+// pair kernels' gathers.  (The field's blocks, 8 KB of queue each, take what is left: in FP32,
+// at the smallest split, seven of the eight that its registers allow.)
 static int smem_split(size_t plane) {
   const size_t need = plane + 8 * sizeof(PairQueue) + 3 * 1024;   // 1 KB of each block is the system's
   for (int kb : {64, 100, 132, 164, 196})
@@ -1102,7 +1104,7 @@ static void fft_convolution(Handle &h, typename Vec2<S>::type *grid, const typen
     else fft_planes<S, false>(h, pl, grid, twiddle, true);
     return;
   }
-  // Any other length (a prime factor above 7, or beyond 256): five per-axis passes.
+  // A length without the two factors, or a plane beyond one CTA: five per-axis passes.
   double *plane = h.d_grid_planes();
   auto run = [&](int d, int sign, bool fuse, bool fromd) {
     const FftAxis &a = h.axes[d];
