@@ -838,10 +838,12 @@ static size_t fft_z_smem(const FftPlan &p, size_t value) { return (2 * (size_t)k
 // barriers, a larger plane the L1 of the kernels beside it (smem_split).  Device time of an
 // evaluation with that limit at 160 / 120 / 100 / 60 KB: 24,000 atoms FP64 2,042 / 1,787 /
 // 1,799 / 1,899 us, 81,000 mixed 3,841 / 3,481 / 3,421 / 3,553.  A plane that they do not
-// (its second axis' lines alone take that much) goes in as few as fit, three or more.  An
-// evaluation with at least 1 / 3 / 5 / 9 chunks there, 10,125 atoms: 80^3 FP64 1,221 / 1,232 /
-// 1,217 / 1,314 us, 96^3 FP64 1,361 / 1,360 / 1,380 / 1,516, 128^3 mixed 1,357 / 1,344 /
-// 1,378 / 1,426; a batch of twelve 3,000-atom boxes at 80^3 FP64 9,395 / 8,271 / 7,905 / 8,380.
+// (its second axis' lines alone take that much) goes in nine chunks or the fewest above that
+// fit: fewer leave the kernels beside it less L1, or no room for the vdW block.  Device time
+// with at least 3 / 6 / 9 / 13 chunks there, at water's density: 46,875 atoms at 80^3 FP64 3,702 /
+// 3,186 / 3,193 / 3,235 us, 81,000 at 96^3 FP64 6,576 / 6,116 / 6,171 / 6,173, 151,959 at 120^3
+// mixed 6,901 / 6,898 / 5,989 / 6,035, 273,375 at 144^3 mixed 13,969 / 12,362 / 12,362 / 12,440.
+// (10,125 atoms on such meshes would be 4 to 8% faster with three.)
 static bool plan_fft(const int nf[3], size_t value, FftPlan &p) {
   p = FftPlan{};
   for (int d = 0; d < 3; d++)
@@ -855,7 +857,7 @@ static bool plan_fft(const int nf[3], size_t value, FftPlan &p) {
     }
     return false;
   };
-  if (!fits(1, 8, 100 * 1024) && !fits(3, 16, kMax)) return false;
+  if (!fits(1, 8, 100 * 1024) && !fits(9, 16, kMax)) return false;
   p.by_row_chunk = fast_div(p.row_chunk);
   p.by_col_chunk = fast_div(p.col_chunk);
   return fft_z_smem(p, value) <= kMax;
