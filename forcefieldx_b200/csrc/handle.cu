@@ -679,6 +679,8 @@ static bool branch_recip(const Handle &h) { return h.capturing && !h.vacuum && !
 // ---------------------------------------------------------------------------
 // Evaluation.  emit_front (coordinates .. permanent field) and emit_back (energies,
 // torques, gradient, reductions) are shared by the direct path and the captured graph.
+// Atoms up to which a captured evaluation's vdW branch starts after the field.
+static int vdw_late_atoms(const Handle &h) { return (h.mixed ? 900 : 400) * h.num_sms; }
 static void emit_front(Handle &h, const double *d_xyz) {
   int tk = timer_begin(h, FFXG_STAGE_LISTS);
   launch_on<k_set_flags, 0, 0>(h.rec, 1, 1, 0, h.stream, h.d_flags, h.list_valid ? 0 : FLAG_REBUILD);
@@ -690,10 +692,14 @@ static void emit_front(Handle &h, const double *d_xyz) {
   // assembly and the sums read (emit_back joins it there), is a branch of the graph.  Before
   // a solve it starts after the real-space field: beside the solver it takes idle issue
   // slots, beside the field it takes the field's (172 against 132 us on the 24,000-atom box,
-  // mixed form; 354 against 220 us FP64).  Inside a batch graph the systems are the branches,
-  // and vdW stays in line (measured 16% more systems/s).
+  // mixed form; 354 against 220 us FP64).  With more atoms its one block a SM would outlast the
+  // solver, and it starts at once.  Late / early, ms: FP64 24,000 atoms 1.69 / 1.73, 52,728 3.55 /
+  // 3.59, 65,856 5.15 / 4.91, 648,000 51.5 / 47.8; mixed 24,000 1.15 / 1.18, 81,000 3.31 / 3.35,
+  // 117,912 4.66 / 4.69, 151,959 6.90 / 6.41, 648,000 33.6 / 28.5.
+  // Inside a batch graph the systems are the branches, and vdW stays in line (measured 16% more
+  // systems/s).
   const bool vdw_branch = h.capturing && !h.vacuum && !h.batch_branch;
-  const bool vdw_late = vdw_branch && h.prm.polarization == FFXG_POLAR_MUTUAL;
+  const bool vdw_late = vdw_branch && h.prm.polarization == FFXG_POLAR_MUTUAL && h.n <= vdw_late_atoms(h);
   auto fork_vdw = [&](cudaStream_t from) {
     cudaEventRecord(h.ev_vdw_fork, from);
     cudaStreamWaitEvent(h.vdw_stream, h.ev_vdw_fork, 0);
